@@ -100,6 +100,12 @@ __device__ __forceinline__ float2 cmulc(float2 a, float2 b)
 {
     return make_float2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
 }
+// a * conj(b), rounded as conj(cmul(conj(a), b)) is: an inverse transform with these products gives
+// the bits of a forward one between two conjugations
+__device__ __forceinline__ float2 cmulc_mirror(float2 a, float2 b)
+{
+    return make_float2(fmaf(a.x, b.x, __fmul_rn(a.y, b.y)), fmaf(-a.x, b.y, __fmul_rn(a.y, b.x)));
+}
 __device__ __forceinline__ float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
 
 // Twiddle multiply d * (hi + lo) with the twiddle carried to about 48 bits.  Rounding a
@@ -208,7 +214,7 @@ __device__ __forceinline__ void dft_reg(float2 (&a)[E])
 // engine's slices take the sets in turn, see kTwSets).  `scr(k1, g)` returns
 // the shared-memory slot for the transpose; `sync()` orders the team's shared
 // accesses (a warp barrier when the team is inside one warp, a block barrier
-// otherwise).
+// otherwise).  DIR: -1 forward, +1 inverse, +2 inverse with cmulc_mirror's products (the slice steps).
 template <int N, int G, int DIR, class Scr, class Sync>
 __device__ __forceinline__ void team_fft(float2 (&v)[N / G], int g, const float2* __restrict__ tw, Scr scr,
                                          Sync sync)
@@ -219,7 +225,8 @@ __device__ __forceinline__ void team_fft(float2 (&v)[N / G], int g, const float2
 #pragma unroll
     for (int k1 = 1; k1 < E; k1++) {
         const float2 w = tw[k1 * G + g];
-        v[brev<E>(k1)] = DIR < 0 ? cmul(v[brev<E>(k1)], w) : cmulc(v[brev<E>(k1)], w);
+        float2& x = v[brev<E>(k1)];
+        x = DIR < 0 ? cmul(x, w) : DIR == 2 ? cmulc_mirror(x, w) : cmulc(x, w);
     }
     sync();
 #pragma unroll

@@ -191,10 +191,9 @@ __global__ void __launch_bounds__(L::ROW_THREADS, L::ROW_MINB) k_row_tt(PassArgs
     float2* scr_base = smem + team * L::SCR_STRIDE_ROW;
     auto scr = [scr_base](int k1, int q) { return scr_base + k1 * (G + 1) + q; };
     auto sync = []() { __syncwarp(); };
-    // inverse row FFT as conj(FFT(conj(x)))
-    conj_all(v);
-    team_fft<N, G, -1>(v, g, tw, scr, sync);
-    conj_all(v);
+    // a true inverse transform: as conj(FFT(conj(x))) the sign changes cost 64 instructions a thread
+    // that packed sums cannot absorb (1024^2, 8 waves: 31.9 -> 31.5 us, wide tiles 38.1 -> 35.1)
+    team_fft<N, G, 2>(v, g, tw, scr, sync);
     if (!beyond) {
         const WaveInfo* wi = opaque(a.waves + b);
         const size_t voff = ((size_t)(a.slice - a.sV_slice_base) * ny + r) * N + g;
@@ -501,14 +500,8 @@ __global__ void __launch_bounds__(L::COL_THREADS, L::COL_MINB)
     auto scr = [scr_base](int k1, int q) { return scr_base + k1 * (G + 1) + q; };
     auto sync = []() { __syncthreads(); };
     const size_t cs = (size_t)G * nx;
-#pragma unroll 1
-    for (int pass = 0; pass < 2; pass++) {
-        team_fft<N, G, -1>(v, g, twp, scr, sync);
-        if (pass == 1) {
-            conj_all(v);
-            break;
-        }
-        if (final_step) break;
+    team_fft<N, G, -1>(v, g, twp, scr, sync);
+    if (!final_step) {
         const float2* pp = opaque(prop_set(wi.prop ? wi.prop : a.prop, a) + (size_t)g * nx + col);
         const uint64_t pl = l2_policy_evict_last();
         if (a.flags & PF_CONJ_PROP) {
@@ -518,7 +511,7 @@ __global__ void __launch_bounds__(L::COL_THREADS, L::COL_MINB)
 #pragma unroll
             for (int j = 0; j < E; j++) v[j] = cmul(v[j], ld_nc_l2hint(pp + j * cs, pl));
         }
-        conj_all(v);
+        team_fft<N, G, 2>(v, g, twp, scr, sync);
     }
     float2* cp = opaque(a.psi + (size_t)b * N * nx + (size_t)g * nx + col);
     const uint64_t pol = l2_policy_wave(a.l2_mode);
@@ -582,14 +575,8 @@ __global__ void __launch_bounds__(256, 2) k_col_step_warp(PassArgs a, const __gr
     auto sync = []() { __syncwarp(); };
     const float2* tw = tw_set<N>(a);   // through L1
     const int col = col0 + w;
-#pragma unroll 1
-    for (int pass = 0; pass < 2; pass++) {
-        team_fft<N, G, -1>(v, lane, tw, scr, sync);
-        if (pass == 1) {
-            conj_all(v);
-            break;
-        }
-        if (final_step) break;
+    team_fft<N, G, -1>(v, lane, tw, scr, sync);
+    if (!final_step) {
         const float2* pp = opaque(prop_set(a.propT, a) + (size_t)col * N + lane);
         const uint64_t pl = l2_policy_evict_last();
         if (a.flags & PF_CONJ_PROP) {
@@ -599,7 +586,7 @@ __global__ void __launch_bounds__(256, 2) k_col_step_warp(PassArgs a, const __gr
 #pragma unroll
             for (int j = 0; j < E; j++) v[j] = cmul(v[j], ld_nc_l2hint(pp + G * j, pl));
         }
-        conj_all(v);
+        team_fft<N, G, 2>(v, lane, tw, scr, sync);
     }
     __syncthreads();   // every warp is done with its scratch: the region takes the result tile
 #pragma unroll

@@ -188,9 +188,7 @@ __global__ void __launch_bounds__(EngineLayout<N>::THREADS, EngineLayout<N>::MIN
                 float2* scr_base = smem + team * L::SCR_STRIDE_ROW;
                 auto scr = [scr_base](int k1, int q) { return scr_base + k1 * (G + 1) + q; };
                 auto sync = []() { __syncwarp(); };
-                conj_all(v);
-                team_fft<N, G, -1>(v, g, tw, scr, sync);
-                conj_all(v);
+                team_fft<N, G, 2>(v, g, tw, scr, sync);
                 {
                     const int r = (dec(3) * SUB + k) * EL::ROWS + team;
                     const WaveInfo* wi = opaque(a.waves + dec(0));
@@ -257,22 +255,16 @@ __global__ void __launch_bounds__(EngineLayout<N>::THREADS, EngineLayout<N>::MIN
                 auto scr = [scr_base](int k1, int q) { return scr_base + k1 * (G + 1) + q; };
                 auto sync = []() { __syncthreads(); };
                 const size_t cs = (size_t)G * N;
-#pragma unroll 1
-                for (int pass = 0; pass < 2; pass++) {
-                    team_fft<N, G, -1>(v, g, tw, scr, sync);
-                    if (pass == 1) {
-                        conj_all(v);
-                        break;
-                    }
-                    const WaveInfo* wi = opaque(a.waves + dec(0));
-                    if (dec(1) == wi->n_slices - 1) break;   // the wave's last slice: no propagation
+                team_fft<N, G, -1>(v, g, tw, scr, sync);
+                const WaveInfo* wi = opaque(a.waves + dec(0));
+                if (dec(1) != wi->n_slices - 1) {   // the wave's last slice is not propagated
                     const int col = (dec(3) * SUB + k) * TC + c;
                     as.slice = dec(1);
                     const float2* pp = opaque(prop_set(wi->prop ? wi->prop : a.prop, as) + (size_t)g * N + col);
                     const uint64_t pl = l2_policy_evict_last();
 #pragma unroll
                     for (int q = 0; q < E; q++) v[q] = cmul(v[q], ld_nc_l2hint(pp + q * cs, pl));
-                    conj_all(v);
+                    team_fft<N, G, 2>(v, g, tw, scr, sync);
                 }
                 const int col = (dec(3) * SUB + k) * TC + c;
                 float2* cp = opaque(a.psi + (size_t)dec(0) * N * N + (size_t)g * N + col);
