@@ -66,7 +66,7 @@ enum ColOp {
 enum PassFlags {
     PF_VACUUM_BEYOND = 1,  // slices past a wave's own count are empty (t = 1) instead of skipped
     PF_ACCUMULATE = 2,     // ROW_INV_ABS2 adds into its output
-    PF_FILTER_AUX = 4,     // COL_STEP also writes the annulus-filtered spectrum to aux
+    PF_FILTER_AUX = 4,     // COL_STEP also writes the annulus-filtered spectrum to aux (aux_stride per wave)
     PF_PROP_ALWAYS = 8,    // COL_STEP propagates even after the wave's last slice
     PF_STORE_X = 16,       // ROW_INV_T_FWD also writes the transmitted real-space wave to xs
     PF_CONJ_PROP = 32,     // COL_STEP multiplies by conj(P) (the adjoint step)
@@ -78,6 +78,7 @@ enum PassFlags {
 struct PassArgs {
     float2* psi;            // [B][ny][nx]
     float2* aux;            // [B][ny][nx] (filtered branch, complex outputs)
+    int64_t aux_stride;     // PF_FILTER_AUX: elements between two waves' filtered spectra in aux
     float* out_real;        // [B][ny][nx] or a frame
     const WaveInfo* waves;  // [B]
     int slice;

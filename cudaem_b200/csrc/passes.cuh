@@ -128,13 +128,12 @@ __global__ void __launch_bounds__(FftLayout<N>::ROW_THREADS, FftLayout<N>::ROW_M
         for (int j = 0; j < E; j++) a.psi[row_off + g + G * j] = v[j];
         return;
     } else {
-        const float2* src = (OP == ROW_INV_ABS2 && (a.flags & PF_FILTER_AUX)) ? a.aux : a.psi;
 #pragma unroll
-        for (int j = 0; j < E; j++) v[j] = src[row_off + g + G * j];
+        for (int j = 0; j < E; j++) v[j] = a.psi[row_off + g + G * j];
         team_fft<N, G, +1>(v, g, tw, scr, sync);
     }
     if (OP == ROW_INV_ABS2) {
-        float* o = a.out_real + ((a.flags & PF_FILTER_AUX) ? (size_t)r * N : row_off);
+        float* o = a.out_real + row_off;
         const float w = wi.weight;
 #pragma unroll
         for (int j = 0; j < E; j++) {
@@ -330,7 +329,7 @@ __global__ void __launch_bounds__(FftLayout<N>::COL_THREADS, FftLayout<N>::COL_M
                 }
             }
             if (a.flags & PF_FILTER_AUX) {
-                float2* ab = opaque(a.aux + (size_t)b * N * nx + (size_t)g * nx + col);
+                float2* ab = opaque(a.aux + (size_t)b * a.aux_stride + (size_t)g * nx + col);
 #pragma unroll
                 for (int j = 0; j < E; j++) {
                     const int k = g + G * j;
@@ -452,8 +451,9 @@ __global__ void __launch_bounds__(FftLayout<N>::COL_THREADS, FftLayout<N>::COL_M
 // shared memory than the classic kernel.  Compared with one 8-byte load per element and thread,
 // the copy engine moves the tile in large requests and leaves the load/store unit free.  The wait
 // for the tile is bounded (PassArgs.wait_cycles): when it runs out the block records the failure
-// in PassArgs.err and returns.  The arithmetic is k_col's COL_STEP.
-template <int N, class L = FftLayout<N>>
+// in PassArgs.err and returns.  The arithmetic is k_col's COL_STEP.  FILT: the propagated spectrum
+// inside the annulus is also written to PassArgs.aux (PF_FILTER_AUX, the thickness series).
+template <int N, class L = FftLayout<N>, bool FILT = false>
 __global__ void __launch_bounds__(L::COL_THREADS, L::COL_MINB)
     k_col_step_tma(PassArgs a, const __grid_constant__ CUtensorMap tmap)
 {
@@ -510,6 +510,14 @@ __global__ void __launch_bounds__(L::COL_THREADS, L::COL_MINB)
         } else {
 #pragma unroll
             for (int j = 0; j < E; j++) v[j] = cmul(v[j], ld_nc_l2hint(pp + j * cs, pl));
+        }
+        if constexpr (FILT) {
+            float2* ab = opaque(a.aux + (size_t)b * a.aux_stride + (size_t)g * nx + col);
+#pragma unroll
+            for (int j = 0; j < E; j++) {
+                const float g2 = det_g2(col, g + G * j, nx, N, a.grid.dgx_f, a.grid.dgy_f);
+                ab[j * cs] = (a.filt_g2in <= g2 && g2 <= a.filt_g2out) ? v[j] : make_float2(0.0f, 0.0f);
+            }
         }
         team_fft<N, G, 2>(v, g, twp, scr, sync);
     }
@@ -621,7 +629,7 @@ static bool col_step_warp(const PassArgs& a, int nwaves, int nx, cudaStream_t st
     }
 }
 
-template <int N, class L = FftLayout<N>>
+template <int N, class L = FftLayout<N>, bool FILT = false>
 static bool col_step_tma(const PassArgs& a, int nwaves, int nx, cudaStream_t st)
 {
     if constexpr (N < 256) {
@@ -631,8 +639,8 @@ static bool col_step_tma(const PassArgs& a, int nwaves, int nx, cudaStream_t st)
         CUtensorMap map;
         if (!encode_wave_tile_map(&map, a.psi, nx, (int64_t)nwaves * N, 2 * L::TC, N < 256 ? N : 256)) return false;
         const size_t sm = L::COL_SMEM + 128;
-        smem_attr(k_col_step_tma<N, L>, sm);
-        k_col_step_tma<N, L><<<(unsigned)(nwaves * (nx / L::TC)), L::COL_THREADS, sm, st>>>(a, map);
+        smem_attr(k_col_step_tma<N, L, FILT>, sm);
+        k_col_step_tma<N, L, FILT><<<(unsigned)(nwaves * (nx / L::TC)), L::COL_THREADS, sm, st>>>(a, map);
         return true;
     }
 }
@@ -1109,6 +1117,11 @@ void col_dispatch(int op, const PassArgs& a, int nwaves, int nx, cudaStream_t st
         if ((a.tile & TILE_WARP_COLS) && col_step_warp<N>(a, nwaves, nx, st)) return;
         if ((a.tile & TILE_NARROW_COLS) && col_step_tma<N, NarrowLayout<N>>(a, nwaves, nx, st)) return;
         if (col_step_tma<N>(a, nwaves, nx, st)) return;
+    } else if (op == COL_STEP && a.variant != PASS_PIPELINED) {
+        // the filtered step of the thickness series: a few waves, so narrow tiles unless wide ones
+        // were found faster for this grid and batch
+        if ((a.tile & TILE_NARROW_COLS) && col_step_tma<N, NarrowLayout<N>, true>(a, nwaves, nx, st)) return;
+        if (col_step_tma<N, FftLayout<N>, true>(a, nwaves, nx, st)) return;
     }
     dim3 grid((unsigned)(nwaves * (nx / L::TC))), block(L::COL_THREADS);
     size_t sm = L::COL_SMEM;
