@@ -24,8 +24,8 @@ REF_TREE = "/root/reference"
 
 def build() -> str:
     subprocess.run(["make", "-C", HERE, "-s"], check=True)
-    if os.path.isdir(REF_TREE):
-        # the reference's own kernels: built only where the reference tree exists
+    if os.path.exists(os.path.join(REF_TREE, "device_kernels.cuh")):
+        # the reference's own kernels: built only where the reference's headers are
         subprocess.run(["make", "-C", HERE, "-s", "ref", f"REF={REF_TREE}"], check=True)
     return LIB_PATH
 
