@@ -313,30 +313,37 @@ size_t col_smem(int N)
 // restructured as atom-culled 64x16 pixel tiles with float4 stores
 // ---------------------------------------------------------------------------
 constexpr int kPotTX = 64, kPotTY = 32, kPotThreads = 256;
-constexpr int kPotRowsPerThread = kPotTY / (kPotThreads / (kPotTX / 4));   // 2 rows of 4 pixels
+constexpr int kPotBlocks = 8;   // per SM; 6 and 5 blocks (40, 48 registers) were slower: 8.5 and 9.1 against 8.1 ms below
+constexpr int kPotSX = 2, kPotSY = 4;   // 8 x 4 pixel slots of a warp's 16 x 16 block, in x and y
 
+// Index of unrolledBinarySearch_c_nR (basic_functions_dev.cuh:47-67): the largest node i <= nR-2 with
+// R2[i] <= r2 (or 0).  The nodes are log-spaced, so the index is the floor of log2(r2) on the node
+// scale; a guess off by one (r2 within the log2 rounding, ~1e-6, of a node) evaluates the
+// neighbouring cubic a hair outside its interval, which the Hermite spline's continuity of value and
+// slope makes equal to 1e-12 (the last node carries its own value and slope).  The floor is taken by
+// adding 1.5 * 2^23 (rounding x - 1/2 to an integer) instead of a conversion, which shares the
+// quarter-rate unit with the logarithm.  The result is masked to the table: lanes beyond the cut-off
+// evaluate too, their value is not used.  log2(0) = -inf becomes node 0.
+__device__ __forceinline__ int spline_node(const ElemTable& T, float r2)
+{
+    float l2;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l2) : "f"(r2));
+    const float x = fmaxf(fmaf(l2, T.inv_dl, T.l0s - 0.5f), -0.25f);
+    return __float_as_int(x + 12582912.0f) & (MS_NR - 1);
+}
 __device__ __forceinline__ float spline_eval(const ElemTable& T, float r2)
 {
-    // index of unrolledBinarySearch_c_nR (basic_functions_dev.cuh:47-67): the largest node
-    // i <= nR-2 with R2[i] <= r2 (or 0).  The nodes are log-spaced, so the index is the floor of
-    // log2(r2) on the node scale; a guess off by one (r2 within the log2 rounding, ~1e-6, of a
-    // node) evaluates the neighbouring cubic a hair outside its interval, which the Hermite
-    // spline's continuity of value and slope makes equal to 1e-12.
-    // log2(r2) for r2 = 0 is -inf, which the floor conversion and the clamp turn into node 0
-    int i = __float2int_rd(fmaf(__log2f(r2), T.inv_dl, T.l0s));
-    i = min(max(i, 0), MS_NR - 2);
-    float d = r2 - T.R2[i];
+    const int i = spline_node(T, r2);
+    const float d = r2 - T.R2[i];
     const ElemCoef4 c = T.c[i];
     return ((c.c3 * d + c.c2) * d + c.c1) * d + c.c0;  // get_value_Cubic_Spline
 }
 
-
 // the same with the cubic coefficients read from a per-pair table (fine slicing)
 __device__ __forceinline__ float spline_eval_c(const ElemTable& T, const float4* __restrict__ coef, float r2)
 {
-    int i = __float2int_rd(fmaf(__log2f(r2), T.inv_dl, T.l0s));
-    i = min(max(i, 0), MS_NR - 2);
-    float d = r2 - T.R2[i];
+    const int i = spline_node(T, r2);
+    const float d = r2 - T.R2[i];
     const float4 c = __ldg(coef + i);
     return ((c.w * d + c.z) * d + c.y) * d + c.x;
 }
@@ -378,17 +385,20 @@ __device__ __forceinline__ int cell_pieces(float lo, float hi, float L, int nc, 
     return n;
 }
 
+// What bounds it: issue slots (88 % busy) and shared-memory reads of the spline table (75 %), not
+// memory.  Of 8.05 ms for 8 x 240 slices of 1024^2 (Si, 1.36 A slices; 9.56 ms with 16 x 8 pixel slots,
+// converted indexes and a shared prefix sum), 2.1 ms are the stores (16 GB, near the memory's rate), 1.6 the
+// tile's atom lookup and 4.3 the splines: 2.4 evaluations per pixel where 1.9 lie inside a disc.
 // WRAP is the periodic wrap of the specimen (a.wrap), a template argument so that the
 // non-periodic kernel carries none of the per-image lookup code
 template <bool FINE, bool WRAP>
-__global__ void __launch_bounds__(kPotThreads, 8) k_potential(PotArgs a)
+__global__ void __launch_bounds__(kPotThreads, kPotBlocks) k_potential(PotArgs a)
 {
     extern __shared__ __align__(16) unsigned char psm[];
     ElemTable* el = reinterpret_cast<ElemTable*>(psm);
     float4* cand = reinterpret_cast<float4*>(psm + sizeof(ElemTable) * a.n_elem);
     unsigned* candp = reinterpret_cast<unsigned*>(cand + kPotThreads);   // fine slicing: pair index
-    __shared__ int wsum[kPotThreads / 32];
-    __shared__ int total_s;
+    __shared__ __align__(16) int wsum[kPotThreads / 32];
     // per warp: the candidates whose disc reaches the warp's 16 x 16 pixel block (indices into cand)
     __shared__ unsigned short whit[kPotThreads / 32][kPotThreads];
     __shared__ unsigned r_beg[kPotMaxRanges], r_pre[kPotMaxRanges + 1];
@@ -399,17 +409,18 @@ __global__ void __launch_bounds__(kPotThreads, 8) k_potential(PotArgs a)
     const int sl = a.slice0 + blockIdx.y;
     const int tiles_x = a.nx / kPotTX;
     const int tx0 = (blockIdx.x % tiles_x) * kPotTX, ty0 = (blockIdx.x / tiles_x) * kPotTY;
-    // Each warp owns a compact 16x16-pixel block of the 64x32 tile (4 x 2 blocks), each lane 4 pixels
-    // in x on 2 rows, so a candidate atom far from a warp's block is skipped by the whole warp.
+    // Each warp owns a compact 16x16-pixel block of the 64x32 tile (4 x 2 blocks), so a candidate atom
+    // far from a warp's block is skipped by the whole warp.  The block is walked in slots of 8 x 4
+    // pixels, one pixel per lane: the smaller a slot, the fewer lanes lie outside an atom's disc
+    // when the slot is evaluated.
     const int t = threadIdx.x, wblk = t >> 5, ln = t & 31;
-    const int px = (wblk % 4) * 4 + (ln % 4);          // in units of 4 pixels across the tile
-    const int py = (wblk / 4) * 16 + (ln / 4);         // first row of the lane inside the tile
-    constexpr int RY = kPotRowsPerThread, ROW_STEP = 8;
-    float acc[RY][4];
+    const int px = (wblk % 4) * 16 + (ln & 7);         // the lane's pixel in the first slot
+    const int py = (wblk / 4) * 16 + (ln >> 3);
+    float acc[kPotSY][kPotSX];
 #pragma unroll
-    for (int r = 0; r < RY; r++)
+    for (int r = 0; r < kPotSY; r++)
 #pragma unroll
-        for (int k = 0; k < 4; k++) acc[r][k] = 0.f;
+        for (int k = 0; k < kPotSX; k++) acc[r][k] = 0.f;
 
     if (sl < a.ns[conf]) {
         {
@@ -498,8 +509,9 @@ __global__ void __launch_bounds__(kPotThreads, 8) k_potential(PotArgs a)
             const unsigned v = vbase + t;
             float4 cv = make_float4(0.f, 0.f, 0.f, 0.f);
             unsigned cpi = 0;
-            int cnt = 0;
-            if (v < n_atoms) {
+            bool near = false;
+            // a tile usually has fewer candidates than one warp has lanes: the other warps skip this
+            if (vbase + 32 * wid < n_atoms && v < n_atoms) {
                 int r = 0;
                 while (r + 1 < nr && r_pre[r + 1] <= v) r++;
                 const unsigned i = r_beg[r] + (v - r_pre[r]);
@@ -514,38 +526,27 @@ __global__ void __launch_bounds__(kPotThreads, 8) k_potential(PotArgs a)
                 const float xs = xa + (float)ox * a.lx, ys = ya + (float)oy * a.ly;  // culling only
                 const float dxr = fmaxf(0.f, fmaxf(X0 - xs, xs - X1));
                 const float dyr = fmaxf(0.f, fmaxf(Y0 - ys, ys - Y1));
-                if (dxr * dxr + dyr * dyr < rm * rm) {
-                    cv = make_float4(xa, ya, w, __int_as_float(e | ((ox + 4) << 8) | ((oy + 4) << 12)));
-                    cpi = i;
-                    cnt = 1;
-                }
+                near = dxr * dxr + dyr * dyr < rm * rm;
+                cv = make_float4(xa, ya, w, __int_as_float(e | ((ox + 4) << 8) | ((oy + 4) << 12)));
+                cpi = i;
             }
             // ordered compaction (deterministic: cell order, then atom order)
-            int incl = cnt;
+            const unsigned nm = __ballot_sync(0xffffffffu, near);
+            if (lane == 0) wsum[wid] = __popc(nm);
+            __syncthreads();
+            int off = 0, total = 0;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                int y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += y;
+            for (int w = 0; w < kPotThreads / 32; w++) {
+                const int n = wsum[w];
+                if (w < wid) off += n;
+                total += n;
             }
-            if (lane == 31) wsum[wid] = incl;
-            __syncthreads();
-            if (t == 0) {
-                int run = 0;
-                for (int w = 0; w < kPotThreads / 32; w++) {
-                    int vv = wsum[w];
-                    wsum[w] = run;
-                    run += vv;
-                }
-                total_s = run;
-            }
-            __syncthreads();
-            const int off = wsum[wid] + incl - cnt;
-            if (cnt > 0) {
+            if (near) {
+                off += __popc(nm & ((1u << lane) - 1u));
                 cand[off] = cv;
                 if (FINE) candp[off] = cpi;
             }
             __syncthreads();
-            const int total = total_s;
             // The warp's own list, one candidate per lane: an atom whose disc misses the warp's 16 x 16
             // pixel block is dropped here (its spline evaluations would all be masked off, yet a
             // divergent warp still issues them), so the loop below runs over hits only.
@@ -574,54 +575,55 @@ __global__ void __launch_bounds__(kPotThreads, 8) k_potential(PotArgs a)
                 const int bits = __float_as_int(cd.w);
                 const ElemTable& T = el[bits & 0xFF];
                 const float rmax2 = T.rmax2;
-                const int ox = ((bits >> 8) & 15) - 4, oy = ((bits >> 12) & 15) - 4;
                 // distance to the image (ox, oy) of the atom: pixel index shifted by -ox*nx, and
                 // i*dx - x formed with dx split in two floats, so the offset is accurate to its own
                 // rounding (the pixel coordinate i*dx alone would carry ~1e-6 A of error)
-                const float fx0 = (float)(tx0 + 4 * px - ox * a.nx), fy0 = (float)(ty0 + py - oy * a.ny);
-                float dx2[4], dy2[RY];
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    const float fx = fx0 + (float)k;
-                    const float d = fmaf(fx, a.dx_lo, fmaf(fx, a.dx_hi, -cd.x));
-                    dx2[k] = d * d;
+                float fx0 = (float)(tx0 + px), fy0 = (float)(ty0 + py);
+                if constexpr (WRAP) {
+                    fx0 -= (float)((((bits >> 8) & 15) - 4) * a.nx);
+                    fy0 -= (float)((((bits >> 12) & 15) - 4) * a.ny);
                 }
+                // squared offsets of the two slot columns and the four slot rows, two at a time
+                const float2 hx = make_float2(a.dx_hi, a.dx_hi), lx = make_float2(a.dx_lo, a.dx_lo);
+                const float2 hy = make_float2(a.dy_hi, a.dy_hi), ly = make_float2(a.dy_lo, a.dy_lo);
+                const float2 fx = make_float2(fx0, fx0 + 8.0f);
+                const float2 fya = make_float2(fy0, fy0 + 4.0f), fyb = make_float2(fy0 + 8.0f, fy0 + 12.0f);
+                const float2 mx = make_float2(-cd.x, -cd.x), my = make_float2(-cd.y, -cd.y);
+                float2 dx2 = __ffma2_rn(fx, lx, __ffma2_rn(fx, hx, mx));
+                float2 dya = __ffma2_rn(fya, ly, __ffma2_rn(fya, hy, my));
+                float2 dyb = __ffma2_rn(fyb, ly, __ffma2_rn(fyb, hy, my));
+                dx2 = __fmul2_rn(dx2, dx2);
+                dya = __fmul2_rn(dya, dya);
+                dyb = __fmul2_rn(dyb, dyb);
 #pragma unroll
-                for (int r = 0; r < RY; r++) {
-                    const float fy = fy0 + (float)(r * ROW_STEP);
-                    const float d = fmaf(fy, a.dy_lo, fmaf(fy, a.dy_hi, -cd.y));
-                    dy2[r] = d * d;
-                }
+                for (int r = 0; r < kPotSY; r++) {
 #pragma unroll
-                for (int r = 0; r < RY; r++) {
-#pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        const float r2 = dx2[k] + dy2[r];
-                        if (r2 < rmax2) {
-                            if (FINE) acc[r][k] += cd.z * spline_eval_c(T, a.pair_coef + (size_t)candp[q] * MS_NR, r2);
-                            else acc[r][k] += cd.z * spline_eval(T, r2);
+                    for (int k = 0; k < kPotSX; k++) {
+                        const float r2 = (k ? dx2.y : dx2.x) + (r == 0 ? dya.x : r == 1 ? dya.y : r == 2 ? dyb.x : dyb.y);
+                        const bool in = r2 < rmax2;
+                        if (__any_sync(0xffffffffu, in)) {
+                            float v;
+                            if (FINE) v = spline_eval_c(T, a.pair_coef + (size_t)candp[q] * MS_NR, r2);
+                            else v = spline_eval(T, r2);
+                            if (in) acc[r][k] += cd.z * v;
                         }
                     }
                 }
             }
-            __syncthreads();
+            if (vbase + kPotThreads < n_atoms) __syncthreads();   // the lists are refilled
         }
     }
+    const int64_t o0 = (int64_t)conf * a.V_conf_stride + (int64_t)(sl - a.V_slice_base) * a.nx * a.ny +
+                       (int64_t)(ty0 + py) * a.nx + tx0 + px;
 #pragma unroll
-    for (int r = 0; r < RY; r++) {
-        const int64_t o = (int64_t)conf * a.V_conf_stride + (int64_t)(sl - a.V_slice_base) * a.nx * a.ny +
-                          (int64_t)(ty0 + py + r * ROW_STEP) * a.nx + tx0 + 4 * px;
-        if (a.T) {
-            // the transmission function t = exp(i V) of the four pixels, as the row pass would form it
+    for (int r = 0; r < kPotSY; r++) {
+#pragma unroll
+        for (int k = 0; k < kPotSX; k++) {
+            const int64_t o = o0 + (int64_t)(4 * r) * a.nx + 8 * k;
+            // the transmission function t = exp(i V) of the pixel, as the row pass would form it
             // (transmission_function.cuh:107-119), so the slice passes read t instead of V
-            float2 t[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++) t[k] = expi_tab(acc[r][k], a.exptab);
-            float4* out = reinterpret_cast<float4*>(a.T + o);
-            out[0] = make_float4(t[0].x, t[0].y, t[1].x, t[1].y);
-            out[1] = make_float4(t[2].x, t[2].y, t[3].x, t[3].y);
-        } else {
-            *reinterpret_cast<float4*>(a.V + o) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+            if (a.T) a.T[o] = expi_tab(acc[r][k], a.exptab);
+            else a.V[o] = acc[r][k];
         }
     }
 }
