@@ -143,6 +143,33 @@ __device__ __forceinline__ void tma_store_commit_and_wait()
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
+// ---------------------------------------------------------------------------
+// Programmatic dependent launch: a step of a small batch is launched before the step ahead of it has
+// ended; it does its setup, then waits (griddepcontrol.wait) until that step's grid has completed and
+// its memory is visible.  Every block waits before it touches the wave and before it returns, so a
+// completed step implies that all steps before it have completed.  The step ahead lets the next one
+// in once its blocks have only their stores left; earlier (at the start) the next steps' blocks crowd
+// the SMs that finish first.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// kern<<<grid, block, smem, st>>>(args...), behind the kernel ahead of it when `chained`
+template <class... KA, class... A>
+inline void launch_step(void (*kern)(KA...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, bool chained,
+                        const A&... args)
+{
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = chained ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kern, args...);   // a failure is read by check_launch
+}
 // default limit of a device-side wait: about one second at the B200's clock
 constexpr long long kWaitCycles = 2000000000LL;
 

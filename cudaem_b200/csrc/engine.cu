@@ -710,6 +710,12 @@ int l2_mode_for_waves(int nwaves, int64_t N)
     return (double)nwaves * (double)N * sizeof(float2) <= 72.0 * 1024 * 1024 ? L2_WAVES_RESIDENT : L2_DEFAULT;
 }
 
+// Whether the slice steps of a batch are launched chained (launch_step): batches so small that the
+// launch latency between two steps shows, up to 2^19 wave pixels.  Per slice, plain and chained:
+// 1 x 256^2 6.74 and 5.84 us, 8 x 256^2 8.49 and 8.23, 1 x 512^2 11.56 and 10.54; but 1 x 1024^2
+// 15.9 and 16.4 (the next step's blocks land unevenly on the SMs), 64 x 1024^2 515 and 521.
+bool chain_steps(const ms_ctx* c, int nwaves, int64_t N) { return !c->profile && nwaves * N <= (1 << 19); }
+
 // Tile shape of the hot passes (row step on the transmission store, column step) for a batch of
 // nw waves on an nx x ny grid: forced by ms_set_tile_shape, else the fastest of the four
 // combinations of wide and narrow row and column tiles, timed on the call's own transmission store
@@ -1107,16 +1113,19 @@ void sim_tem_like(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* o
         // tilt) runs as separate passes and the engine takes the slices after it
         const bool eng = engine_fits(c, p.nx, p.ny, pa.flags);
         const int sl_end = eng ? (plane ? std::min(1, S_max) : 0) : S_max;
+        const bool chain = pc.ev.size() <= 1 && chain_steps(c, nw, N);
         auto slices = [&] {
             PassArgs q = pa;
             for (int sl = 0; sl < sl_end; sl++) {
                 pc.wait(c, sl);
                 q.slice = sl;
                 q.tw = s.tw_x;
+                q.chained = chain && sl > 0;   // the first step follows copies
                 PassArgs pr = q;
                 if (sl == 0 && iw == MS_IW_PLANE_TILTED) pr.flags |= PF_TILT_INCIDENT;
                 run_row(c, p.nx, (sl == 0 && plane) ? ROW_T_FWD : ROW_INV_T_FWD, pr, nw, p.ny, st);
                 q.tw = s.tw_y;
+                q.chained = chain;
                 PassArgs pq = q;
                 if (c->inject == MS_INJECT_WAIT_TIMEOUT) pq.flags |= PF_TEST_WAIT;
                 run_col(c, p.ny, COL_STEP, pq, nw, p.nx, st);
@@ -1574,6 +1583,7 @@ void sim_stem(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* out)
                         q.tw = s.tw_x;
                         timed(c, "engine", [&] { engine_launch(q, e, p.nx, nb, st); });
                     }
+                    q.chained = chain_steps(c, nb, N);   // the first step follows the probe's kernel
                     for (int sl = 0; sl < (eng ? 0 : S); sl++) {
                         q.slice = sl;
                         q.tw = s.tw_x;
@@ -1700,6 +1710,7 @@ void sim_thickness(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* 
         pa.filt_g2out = g2out;
         pa.tile = choose_tile(c, pa, p.nx, p.ny, nw, g.S_cap, st);
         c->last_tile = pa.tile;
+        const bool chain = chain_steps(c, nw, N);
         auto slices = [&] {
             PassArgs q = pa;
             if (iw == MS_IW_CONVERGENT) {
@@ -1713,7 +1724,9 @@ void sim_thickness(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* 
                     q.flags = PF_VACUUM_BEYOND;
                     q.tw = s.tw_x;
                     if (sl == 0 && iw == MS_IW_PLANE_TILTED) q.flags |= PF_TILT_INCIDENT;
+                    q.chained = chain && sl > 0;   // the first step follows copies
                     run_row(c, p.nx, (sl == 0 && iw != MS_IW_CONVERGENT) ? ROW_T_FWD : ROW_INV_T_FWD, q, nw, p.ny, st);
+                    q.chained = chain;
                     q.flags = PF_VACUUM_BEYOND | PF_PROP_ALWAYS | PF_FILTER_AUX;
                     q.aux = aux + (int64_t)(sl - s0) * N;
                     q.tw = s.tw_y;
@@ -1824,8 +1837,13 @@ void sim_stem_forward_potential(ms_ctx* c, const ms_params& p, const float* V, i
         CK(cudaMemcpyAsync(dwv, wv.data(), sizeof(WaveInfo) * nb, cudaMemcpyHostToDevice, st));
         float2* psi = (float2*)c->buf("psi", sizeof(float2) * N * B);
         PassArgs pa = pass_args(s, psi, dwv, sV, slot, cond);
+        // the tile shape is tuned as for the simulations, and the waves stay in L2 where they fit
+
+        pa.l2_mode = l2_mode_for_waves(nb, N);
+        pa.tile = choose_tile(c, pa, p.nx, p.ny, nb, S, st);
         pa.tw = s.tw_y;
         run_col(c, p.ny, COL_PROBE_INV, pa, nb, p.nx, st);
+        pa.chained = chain_steps(c, nb, N);
         for (int sl = 0; sl < S; sl++) {
             pa.slice = sl;
             pa.tw = s.tw_x;
@@ -1924,6 +1942,8 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
         WaveInfo* dwv = (WaveInfo*)c->buf("waves", sizeof(WaveInfo) * B);
         CK(cudaMemcpyAsync(dwv, wv.data(), sizeof(WaveInfo) * nb, cudaMemcpyHostToDevice, st));
         PassArgs pa = pass_args(s, adj, dwv, sV, slot, cond);
+        pa.l2_mode = l2_mode_for_waves(nb, N);
+        pa.tile = choose_tile(c, pa, p.nx, p.ny, nb, S, st);
         pa.det_thr = dthr;
         pa.ndet = ndet;
         pa.resid = resid;

@@ -170,6 +170,7 @@ __global__ void __launch_bounds__(L::ROW_THREADS, L::ROW_MINB) k_row_tt(PassArgs
     const int b = blockIdx.x / blocks_per_wave;
     const int team = threadIdx.x / G, g = threadIdx.x % G;
     const int r = (blockIdx.x % blocks_per_wave) * L::ROWS + team;
+    chain_wait();
     const bool beyond = a.slice >= a.waves[b].n_slices;
     if (beyond && !(a.flags & PF_VACUUM_BEYOND)) return;
     float2 v[E];
@@ -213,6 +214,7 @@ __global__ void __launch_bounds__(L::ROW_THREADS, L::ROW_MINB) k_row_tt(PassArgs
         }
     }
     team_fft<N, G, -1>(v, g, tw, scr, sync);
+    chain_trigger();
     float2* dst = opaque(a.psi) + ((size_t)b * ny + r) * N + g;
     const uint64_t pol = l2_policy_wave(MODE);
 #pragma unroll
@@ -472,18 +474,22 @@ __global__ void __launch_bounds__(L::COL_THREADS, L::COL_MINB)
     const int c = threadIdx.x % TC, g = threadIdx.x / TC;
     const int col = col0 + c;
     const WaveInfo& wi = a.waves[b];
-    if (a.slice >= wi.n_slices && !(a.flags & PF_VACUUM_BEYOND)) return;
+    if (a.slice >= wi.n_slices && !(a.flags & PF_VACUUM_BEYOND)) {
+        chain_wait();
+        return;
+    }
     const bool final_step = (a.slice == wi.n_slices - 1) && !(a.flags & PF_PROP_ALWAYS);
     float2* tile = smem;
     float2* tws = smem + TC * L::SCR_STRIDE_COL;
+    if constexpr (!L::NARROW)
+        for (int i = threadIdx.x; i < N; i += blockDim.x) tws[i] = tw_set<N>(a)[i];
+    if (threadIdx.x == 0) mbar_init(&bar, 1);
+    chain_wait();
     if (threadIdx.x == 0) {
-        mbar_init(&bar, 1);
         mbar_expect_tx(&bar, TILE_BYTES + ((a.flags & PF_TEST_WAIT) ? 16u : 0u));
 #pragma unroll
         for (int q = 0; q < N / BOX; q++) tma_load_2d(tile + q * BOX * TC, &tmap, 2 * col0, b * N + q * BOX, &bar);
     }
-    if constexpr (!L::NARROW)
-        for (int i = threadIdx.x; i < N; i += blockDim.x) tws[i] = tw_set<N>(a)[i];
     const float2* twp = L::NARROW ? tw_set<N>(a) : tws;
     __syncthreads();
     const long long limit = (a.flags & PF_TEST_WAIT) ? 2000000LL : (a.wait_cycles > 0 ? a.wait_cycles : kWaitCycles);
@@ -521,6 +527,7 @@ __global__ void __launch_bounds__(L::COL_THREADS, L::COL_MINB)
         }
         team_fft<N, G, 2>(v, g, twp, scr, sync);
     }
+    chain_trigger();
     float2* cp = opaque(a.psi + (size_t)b * N * nx + (size_t)g * nx + col);
     const uint64_t pol = l2_policy_wave(a.l2_mode);
 #pragma unroll
@@ -555,10 +562,14 @@ __global__ void __launch_bounds__(256, 2) k_col_step_warp(PassArgs a, const __gr
     const int col0 = (blockIdx.x % tiles) * TC;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const WaveInfo& wi = a.waves[b];
-    if (a.slice >= wi.n_slices && !(a.flags & PF_VACUUM_BEYOND)) return;
+    if (a.slice >= wi.n_slices && !(a.flags & PF_VACUUM_BEYOND)) {
+        chain_wait();
+        return;
+    }
     const bool final_step = (a.slice == wi.n_slices - 1) && !(a.flags & PF_PROP_ALWAYS);
+    if (threadIdx.x == 0) mbar_init(&bar, 1);
+    chain_wait();
     if (threadIdx.x == 0) {
-        mbar_init(&bar, 1);
         mbar_expect_tx(&bar, TILE_BYTES + ((a.flags & PF_TEST_WAIT) ? 16u : 0u));
 #pragma unroll
         for (int q = 0; q < N / BOX; q++) tma_load_2d(base + q * BOX * 64, &tmap, 2 * col0, b * N + q * BOX, &bar);
@@ -596,6 +607,7 @@ __global__ void __launch_bounds__(256, 2) k_col_step_warp(PassArgs a, const __gr
         }
         team_fft<N, G, 2>(v, lane, tw, scr, sync);
     }
+    chain_trigger();
     __syncthreads();   // every warp is done with its scratch: the region takes the result tile
 #pragma unroll
     for (int j = 0; j < E; j++) *at(lane + G * j, w) = v[j];
@@ -624,7 +636,7 @@ static bool col_step_warp(const PassArgs& a, int nwaves, int nx, cudaStream_t st
         if (!encode_wave_tile_map(&map, a.psi, nx, (int64_t)nwaves * N, 16, 256, true)) return false;
         constexpr size_t sm = sizeof(float2) * 8 * (L::E * (L::G + 1) + 1) + 1024;
         smem_attr(k_col_step_warp<N>, sm);
-        k_col_step_warp<N><<<(unsigned)(nwaves * (nx / 8)), 256, sm, st>>>(a, map);
+        launch_step(k_col_step_warp<N>, (unsigned)(nwaves * (nx / 8)), 256, sm, st, a.chained != 0, a, map);
         return true;
     }
 }
@@ -640,7 +652,8 @@ static bool col_step_tma(const PassArgs& a, int nwaves, int nx, cudaStream_t st)
         if (!encode_wave_tile_map(&map, a.psi, nx, (int64_t)nwaves * N, 2 * L::TC, N < 256 ? N : 256)) return false;
         const size_t sm = L::COL_SMEM + 128;
         smem_attr(k_col_step_tma<N, L, FILT>, sm);
-        k_col_step_tma<N, L, FILT><<<(unsigned)(nwaves * (nx / L::TC)), L::COL_THREADS, sm, st>>>(a, map);
+        launch_step(k_col_step_tma<N, L, FILT>, (unsigned)(nwaves * (nx / L::TC)), L::COL_THREADS, sm, st, a.chained != 0,
+                    a, map);
         return true;
     }
 }
@@ -1042,7 +1055,7 @@ void row_dispatch(int op, const PassArgs& a, int nwaves, int ny, cudaStream_t st
                                                    : k_row_tt<N, L2_DEFAULT, NL>;
         const size_t nsm = sizeof(float2) * (size_t)NL::ROWS * NL::SCR_STRIDE_ROW;
         smem_attr(kern, nsm);
-        kern<<<(unsigned)(nwaves * (ny / NL::ROWS)), NL::ROW_THREADS, nsm, st>>>(a);
+        launch_step(kern, (unsigned)(nwaves * (ny / NL::ROWS)), NL::ROW_THREADS, nsm, st, a.chained != 0, a);
         return;
     }
     if (op == ROW_INV_T_FWD) {
@@ -1055,13 +1068,13 @@ void row_dispatch(int op, const PassArgs& a, int nwaves, int ny, cudaStream_t st
                                                        : k_row_tt<N, L2_DEFAULT, NL, true>;
             const size_t nsm = sizeof(float2) * (size_t)NL::ROWS * NL::SCR_STRIDE_ROW;
             smem_attr(kern, nsm);
-            kern<<<(unsigned)(nwaves * (ny / NL::ROWS)), NL::ROW_THREADS, nsm, st>>>(a);
+            launch_step(kern, (unsigned)(nwaves * (ny / NL::ROWS)), NL::ROW_THREADS, nsm, st, a.chained != 0, a);
         } else {
             auto kern = a.l2_mode == L2_WAVES_RESIDENT ? k_row_tt<N, L2_WAVES_RESIDENT, L, true>
                         : a.l2_mode == L2_SHARED_T     ? k_row_tt<N, L2_SHARED_T, L, true>
                                                        : k_row_tt<N, L2_DEFAULT, L, true>;
             smem_attr(kern, sm);
-            kern<<<grid, block, sm, st>>>(a);
+            launch_step(kern, grid.x, block.x, sm, st, a.chained != 0, a);
         }
         return;
     }
@@ -1095,7 +1108,7 @@ void row_dispatch(int op, const PassArgs& a, int nwaves, int ny, cudaStream_t st
                                                    : (a.l2_mode == L2_SHARED_T ? k_row_tt<N, L2_SHARED_T>
                                                                                : k_row_tt<N, L2_DEFAULT>);
         smem_attr(kern, sm);
-        kern<<<grid, block, sm, st>>>(a);
+        launch_step(kern, grid.x, block.x, sm, st, a.chained != 0, a);
     } break;
     case ROW_TT_FWD:
         smem_attr(k_row<N, ROW_TT_FWD>, sm);
