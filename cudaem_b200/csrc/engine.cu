@@ -1791,6 +1791,20 @@ void sim_potential(ms_ctx* c, const ms_params& p, const ms_atoms& a, int conf, f
 // ---------------------------------------------------------------------------
 // STEM on caller potentials (wave_modulation_batch, wave_function.cuh:74-87)
 // ---------------------------------------------------------------------------
+namespace {
+// The transmission t = exp(iV) of the caller's slices, formed once per call instead of once per
+// probe in the row steps (the same values), or null: with fewer than four probes the extra pass over
+// the slices costs what it saves, and the store may take a quarter of the free memory.  512^2, 16
+// probes: the row step takes 15 us on the store and 25 us on V.
+float2* caller_transmission(ms_ctx* c, const Setup& s, const float* V, int64_t n, int np)
+{
+    if (np < 4 || (double)n * sizeof(float2) > 0.25 * (double)c->free_mem()) return nullptr;
+    float2* T = (float2*)c->buf("caller_t", sizeof(float2) * n);
+    launch_transmission(V, n, s.exptab, T, c->stream);
+    return T;
+}
+}  // namespace
+
 void sim_stem_forward_potential(ms_ctx* c, const ms_params& p, const float* V, int S, int on_dev, double z_init,
                                 const double* xy, int np, float* I)
 {
@@ -1816,6 +1830,7 @@ void sim_stem_forward_potential(ms_ctx* c, const ms_params& p, const float* V, i
     }
     float* dthr = (float*)c->buf("det_thr", sizeof(float) * 2 * ndet);
     CK(cudaMemcpyAsync(dthr, thr.data(), sizeof(float) * 2 * ndet, cudaMemcpyHostToDevice, st));
+    float2* sT = caller_transmission(c, s, sV, slot, np);
     const int B = std::min(np, p.probe_batch > 0 ? p.probe_batch : 256);
     const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>(64, N / 4096));
     double* partial = (double*)c->buf("det_part", sizeof(double) * B * nblk * ndet);
@@ -1837,8 +1852,8 @@ void sim_stem_forward_potential(ms_ctx* c, const ms_params& p, const float* V, i
         CK(cudaMemcpyAsync(dwv, wv.data(), sizeof(WaveInfo) * nb, cudaMemcpyHostToDevice, st));
         float2* psi = (float2*)c->buf("psi", sizeof(float2) * N * B);
         PassArgs pa = pass_args(s, psi, dwv, sV, slot, cond);
+        pa.tt = sT;
         // the tile shape is tuned as for the simulations, and the waves stay in L2 where they fit
-
         pa.l2_mode = l2_mode_for_waves(nb, N);
         pa.tile = choose_tile(c, pa, p.nx, p.ny, nb, S, st);
         pa.tw = s.tw_y;
@@ -1901,6 +1916,7 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
     float* dtgt = (float*)c->buf("adj_target", sizeof(float) * np * ndet);
     CK(cudaMemcpyAsync(dtgt, target, sizeof(float) * np * ndet, cudaMemcpyHostToDevice, st));
 
+    float2* sT = caller_transmission(c, s, sV, slot, np);
     const int k = p.ckpt_interval;
     const int nseg = (S + k - 1) / k;
     // probes per batch: adjoint wave, forward wave, one segment of transmitted waves and the
@@ -1942,6 +1958,7 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
         WaveInfo* dwv = (WaveInfo*)c->buf("waves", sizeof(WaveInfo) * B);
         CK(cudaMemcpyAsync(dwv, wv.data(), sizeof(WaveInfo) * nb, cudaMemcpyHostToDevice, st));
         PassArgs pa = pass_args(s, adj, dwv, sV, slot, cond);
+        pa.tt = sT;
         pa.l2_mode = l2_mode_for_waves(nb, N);
         pa.tile = choose_tile(c, pa, p.nx, p.ny, nb, S, st);
         pa.det_thr = dthr;

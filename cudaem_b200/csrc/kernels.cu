@@ -127,6 +127,22 @@ void launch_prop_table(int nx, int ny, double dgx, double dgy, double g0x, doubl
     check_launch("propagator table");
 }
 
+// One thread per pixel: 4 bytes in, 8 out, coalesced whatever V's alignment; bound by memory (the
+// exponential's table stays in L1).
+__global__ void __launch_bounds__(256) k_transmission(const float* V, int64_t n, const float2* exptab, float2* T)
+{
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        T[i] = expi_tab(__ldg(V + i), exptab);
+}
+
+void launch_transmission(const float* V, int64_t n, const float2* exptab, float2* T, cudaStream_t st)
+{
+    const unsigned blocks = (unsigned)std::min<int64_t>((n + 255) / 256, 32ll * num_sms());
+    k_transmission<<<blocks, 256, 0, st>>>(V, n, exptab, T);
+    count_launch();
+    check_launch("transmission");
+}
+
 void launch_row(int N, int op, const PassArgs& a, int nwaves, int ny, cudaStream_t st)
 {
     if (nwaves <= 0) return;

@@ -48,8 +48,7 @@ enum RowOp {
     ROW_INV_T_FWD = 1,
     ROW_INV_ABS2 = 2,
     ROW_INV_STORE = 3,
-    ROW_ADJ = 4,
-    ROW_INV_T_FWD_X = 5,  // ROW_INV_T_FWD that also keeps t psi in xs (selected by PF_STORE_X)
+    ROW_ADJ = 4,          // the adjoint of ROW_INV_T_FWD
     ROW_INV_TT_FWD = 6,   // ROW_INV_T_FWD with t = exp(i V) read from a transmission store (selected by tt)
     ROW_TT_FWD = 7        // ROW_T_FWD likewise
 };
@@ -204,6 +203,8 @@ void launch_col(int N, int op, const PassArgs& a, int nwaves, int nx, cudaStream
 size_t row_smem(int N);
 size_t col_smem(int N);
 void launch_potential(const PotArgs& a, int n_conf, cudaStream_t st);
+// T[i] = exp(i V[i]), the row steps' values
+void launch_transmission(const float* V, int64_t n, const float2* exptab, float2* T, cudaStream_t st);
 void launch_prop_table(int nx, int ny, double dgx, double dgy, double g0x, double g0y, double w, double alpha,
                        double gl2, int bwl, float2* P, cudaStream_t st, float2* PT = nullptr);
 

@@ -35,6 +35,9 @@ __device__ __forceinline__ const float2* prop_set(const float2* base, const Pass
 }
 
 // ---------------------------------------------------------------------------
+// The row passes off the slice loop: a plane wave's first slice (ROW_T_FWD on a σV store, ROW_TT_FWD on
+// a transmission store: t, then the forward transform) and the image transforms (ROW_INV_ABS2,
+// ROW_INV_STORE).
 template <int N, int OP>
 __global__ void __launch_bounds__(FftLayout<N>::ROW_THREADS, FftLayout<N>::ROW_MINB) k_row(PassArgs a)
 {
@@ -48,91 +51,57 @@ __global__ void __launch_bounds__(FftLayout<N>::ROW_THREADS, FftLayout<N>::ROW_M
     const int r = (blockIdx.x % blocks_per_wave) * L::ROWS + team;
     const WaveInfo wi = a.waves[b];
     const bool beyond = a.slice >= wi.n_slices;
-    constexpr bool kT = OP == ROW_T_FWD || OP == ROW_INV_T_FWD || OP == ROW_INV_T_FWD_X || OP == ROW_INV_TT_FWD ||
-                        OP == ROW_TT_FWD;
-    constexpr bool kTT = OP == ROW_INV_TT_FWD || OP == ROW_TT_FWD;
+    constexpr bool kT = OP == ROW_T_FWD || OP == ROW_TT_FWD;
+    constexpr bool kTT = OP == ROW_TT_FWD;
     if (kT && beyond && !(a.flags & PF_VACUUM_BEYOND)) return;
 
     const size_t row_off = ((size_t)b * ny + r) * N;
     float2 v[E];
-    // the wave's loads go out first, so their latency overlaps the table staging below
-    if (OP == ROW_INV_T_FWD || OP == ROW_INV_T_FWD_X || OP == ROW_INV_TT_FWD || OP == ROW_ADJ) {
-#pragma unroll
-        for (int j = 0; j < E; j++) v[j] = a.psi[row_off + g + G * j];
-    }
     float2* tw = smem + L::ROWS * L::SCR_STRIDE_ROW;
     float2* etab = tw + N;
     for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = tw_set<N>(a)[i];
-    if ((kT && !kTT) || OP == ROW_ADJ)
+    if (kT && !kTT)
         for (int i = threadIdx.x; i < kExpTab; i += blockDim.x) etab[i] = a.exptab[i];
     __syncthreads();
     float2* scr_base = smem + team * L::SCR_STRIDE_ROW;
     auto scr = [scr_base](int k1, int q) { return scr_base + k1 * (G + 1) + q; };
     auto sync = []() { __syncwarp(); };
 
-    if (kT || OP == ROW_ADJ) {
+    if constexpr (kT) {
         const size_t voff = ((size_t)(a.slice - a.sV_slice_base) * ny + r) * N;
         const float* vr = kTT ? nullptr : (wi.sV ? wi.sV : a.sV + (size_t)wi.conf_slot * a.sV_slot_stride) + voff;
         const float2* tr = kTT ? a.tt + (size_t)wi.conf_slot * a.sV_slot_stride + voff : nullptr;
-        if (OP == ROW_T_FWD || OP == ROW_TT_FWD) {
-            if (a.flags & PF_TILT_INCIDENT) {
-                // apply_beam_tilt / exp_r_factor_2d (incident_wave.cuh:72-78, device_kernels.cuh:519-533):
-                // the plane wave exp(2 pi i (g0x Rx + g0y Ry)), R measured from the box centre, phase in FP64
-                const double ry = (double)r * (a.grid.ly / ny) - 0.5 * a.grid.ly;
+        if (a.flags & PF_TILT_INCIDENT) {
+            // apply_beam_tilt / exp_r_factor_2d (incident_wave.cuh:72-78, device_kernels.cuh:519-533):
+            // the plane wave exp(2 pi i (g0x Rx + g0y Ry)), R measured from the box centre, phase in FP64
+            const double ry = (double)r * (a.grid.ly / ny) - 0.5 * a.grid.ly;
 #pragma unroll
-                for (int j = 0; j < E; j++) {
-                    const double rx = (double)(g + G * j) * (a.grid.lx / N) - 0.5 * a.grid.lx;
-                    v[j] = expi_d(6.283185307179586476925 * (a.grid.g0x * rx + a.grid.g0y * ry));
-                }
+            for (int j = 0; j < E; j++) {
+                const double rx = (double)(g + G * j) * (a.grid.lx / N) - 0.5 * a.grid.lx;
+                v[j] = expi_d(6.283185307179586476925 * (a.grid.g0x * rx + a.grid.g0y * ry));
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < E; j++) v[j] = make_float2(1.0f, 0.0f);
+        }
+        if (!beyond) {
+            if constexpr (kTT) {
+#pragma unroll
+                for (int j = 0; j < E; j++) v[j] = cmul(v[j], __ldg(tr + g + G * j));
             } else {
 #pragma unroll
-                for (int j = 0; j < E; j++) v[j] = make_float2(1.0f, 0.0f);
+                for (int j = 0; j < E; j++) v[j] = cmul(v[j], expi_tab(__ldg(vr + g + G * j), etab));
             }
         }
-        // pass 0: inverse row FFT as conj(FFT(conj(x))), then the transmission;
-        // pass 1: forward row FFT.  One copy of the transform code serves both.
-        // ROW_ADJ is the adjoint of the same operator: with xbar the inverse row transform of the
-        // adjoint wave and x = t psi the stored forward wave, dL/dV += Re(i x conj(xbar)) and the
-        // adjoint continues as conj(t) xbar (or_stem_backward's chain, restated per row).
-#pragma unroll 1
-        for (int pass = (OP == ROW_T_FWD || OP == ROW_TT_FWD) ? 1 : 0; pass < 2; pass++) {
-            if (pass == 0) conj_all(v);
-            else if (OP == ROW_ADJ) {
-                // each wave's dL/dV contribution goes to its own plane of a.dV ([B][ny][nx]); the planes
-                // are summed in a fixed order afterwards, so the gradient is reproducible bit for bit
-                const float2* xr = a.xs + row_off;
-                float* gr = a.dV + row_off;
-#pragma unroll
-                for (int j = 0; j < E; j++) {
-                    const float2 x = __ldg(xr + g + G * j);
-                    gr[g + G * j] = x.x * v[j].y - x.y * v[j].x;
-                    v[j] = cmulc(v[j], expi_tab(__ldg(vr + g + G * j), etab));
-                }
-            } else if (!beyond) {
-                if constexpr (kTT) {
-#pragma unroll
-                    for (int j = 0; j < E; j++) v[j] = cmul(v[j], __ldg(tr + g + G * j));
-                } else {
-#pragma unroll
-                    for (int j = 0; j < E; j++) v[j] = cmul(v[j], expi_tab(__ldg(vr + g + G * j), etab));
-                }
-                if constexpr (OP == ROW_INV_T_FWD_X) {
-#pragma unroll
-                    for (int j = 0; j < E; j++) a.xs[row_off + g + G * j] = v[j];
-                }
-            }
-            team_fft<N, G, -1>(v, g, tw, scr, sync);
-            if (pass == 0) conj_all(v);
-        }
+        team_fft<N, G, -1>(v, g, tw, scr, sync);
 #pragma unroll
         for (int j = 0; j < E; j++) a.psi[row_off + g + G * j] = v[j];
         return;
-    } else {
-#pragma unroll
-        for (int j = 0; j < E; j++) v[j] = a.psi[row_off + g + G * j];
-        team_fft<N, G, +1>(v, g, tw, scr, sync);
     }
-    if (OP == ROW_INV_ABS2) {
+#pragma unroll
+    for (int j = 0; j < E; j++) v[j] = a.psi[row_off + g + G * j];
+    team_fft<N, G, +1>(v, g, tw, scr, sync);
+    if constexpr (OP == ROW_INV_ABS2) {
         float* o = a.out_real + row_off;
         const float w = wi.weight;
 #pragma unroll
@@ -141,7 +110,7 @@ __global__ void __launch_bounds__(FftLayout<N>::ROW_THREADS, FftLayout<N>::ROW_M
             if (a.flags & PF_ACCUMULATE) o[g + G * j] += i2;
             else o[g + G * j] = i2;
         }
-    } else if (OP == ROW_INV_STORE) {
+    } else if constexpr (OP == ROW_INV_STORE) {
 #pragma unroll
         for (int j = 0; j < E; j++) a.aux[row_off + g + G * j] = v[j];
     }
@@ -157,10 +126,15 @@ __global__ void __launch_bounds__(FftLayout<N>::ROW_THREADS, FftLayout<N>::ROW_M
 // L is the tile layout: FftLayout<N> (wide, the default) or NarrowLayout<N> (one warp of rows per
 // block, twiddles read from global memory).  SV: the slice is a σV store (the wave's own, WaveInfo.sV,
 // or the configuration's slot of PassArgs.sV) and t = exp(iσV) is formed here from the exp table
-// (read through L1), as k_row's ROW_INV_T_FWD does: the same values as a transmission store.
-// XS (with SV): the transmitted real-space wave t·ψ is also written to PassArgs.xs, as
-// ROW_INV_T_FWD_X does for the adjoint's checkpoints.
-template <int N, int MODE, class L = FftLayout<N>, bool SV = false, bool XS = false>
+// (read through L1): the same values as a transmission store.
+// KEEP_X: the transmitted real-space wave t·ψ is also written to PassArgs.xs (the adjoint's
+// checkpoints).
+// ADJOINT: the adjoint of the same step.  With xbar the inverse row transform of the adjoint wave and
+// x = t psi the stored forward wave, the wave's dL/dV contribution Re(i x conj(xbar)) goes to its own
+// plane of PassArgs.dV ([B][ny][nx]; the planes are summed in a fixed order afterwards, so the gradient
+// is reproducible bit for bit), and the adjoint goes on as conj(t) xbar.
+enum RowForm { ROWF_STEP = 0, ROWF_KEEP_X = 1, ROWF_ADJOINT = 2 };
+template <int N, int MODE, class L = FftLayout<N>, bool SV = false, int FORM = ROWF_STEP>
 __global__ void __launch_bounds__(L::ROW_THREADS, L::ROW_MINB) k_row_tt(PassArgs a)
 {
     constexpr int G = L::G, E = L::E;
@@ -197,20 +171,36 @@ __global__ void __launch_bounds__(L::ROW_THREADS, L::ROW_MINB) k_row_tt(PassArgs
     if (!beyond) {
         const WaveInfo* wi = opaque(a.waves + b);
         const size_t voff = ((size_t)(a.slice - a.sV_slice_base) * ny + r) * N + g;
+        if constexpr (FORM == ROWF_ADJOINT) {
+            const size_t xoff = ((size_t)b * ny + r) * N + g;
+            const float2* xr = opaque(a.xs) + xoff;
+            float* gr = opaque(a.dV) + xoff;
+#pragma unroll
+            for (int j = 0; j < E; j++) {
+                const float2 x = __ldg(xr + G * j);
+                gr[G * j] = x.x * v[j].y - x.y * v[j].x;
+            }
+        }
         if constexpr (SV) {
             const float* vr = (wi->sV ? wi->sV : opaque(a.sV) + (size_t)wi->conf_slot * a.sV_slot_stride) + voff;
 #pragma unroll
-            for (int j = 0; j < E; j++) v[j] = cmul(v[j], expi_tab(__ldg(vr + G * j), a.exptab));
-            if constexpr (XS) {
-                float2* xr = opaque(a.xs) + ((size_t)b * ny + r) * N + g;
-#pragma unroll
-                for (int j = 0; j < E; j++) xr[G * j] = v[j];
+            for (int j = 0; j < E; j++) {
+                const float2 t = expi_tab(__ldg(vr + G * j), a.exptab);
+                v[j] = FORM == ROWF_ADJOINT ? cmulc(v[j], t) : cmul(v[j], t);
             }
         } else {
             const float2* tr = opaque(a.tt) + (size_t)wi->conf_slot * a.sV_slot_stride + voff;
             const uint64_t pol = l2_policy_trans(MODE);
 #pragma unroll
-            for (int j = 0; j < E; j++) v[j] = cmul(v[j], ld_nc_l2hint(tr + G * j, pol));
+            for (int j = 0; j < E; j++) {
+                const float2 t = ld_nc_l2hint(tr + G * j, pol);
+                v[j] = FORM == ROWF_ADJOINT ? cmulc(v[j], t) : cmul(v[j], t);
+            }
+        }
+        if constexpr (FORM == ROWF_KEEP_X) {
+            float2* xr = opaque(a.xs) + ((size_t)b * ny + r) * N + g;
+#pragma unroll
+            for (int j = 0; j < E; j++) xr[G * j] = v[j];
         }
     }
     team_fft<N, G, -1>(v, g, tw, scr, sync);
@@ -1024,96 +1014,72 @@ void row_dispatch(int op, const PassArgs& a, int nwaves, int ny, cudaStream_t st
     if (op == ROW_INV_T_FWD && a.variant == PASS_PIPELINED && !(a.flags & PF_STORE_X) && !a.tt && a.sV &&
         ((uintptr_t)a.sV & 15) == 0 && row_pipe<N>(a, nwaves, ny, st))
         return;
-    dim3 grid((unsigned)(nwaves * (ny / L::ROWS))), block(L::ROW_THREADS);
-    size_t sm = L::ROW_SMEM;
-    if (op == ROW_INV_T_FWD && (a.flags & PF_STORE_X) && !a.tt) {
-        // the adjoint's forward step that keeps t psi: the lean kernel with the extra store
-        if (a.tile & TILE_NARROW_ROWS) {
-            using NL = NarrowLayout<N>;
-            const size_t nsm = sizeof(float2) * (size_t)NL::ROWS * NL::SCR_STRIDE_ROW;
-            smem_attr(k_row_tt<N, L2_DEFAULT, NL, true, true>, nsm);
-            k_row_tt<N, L2_DEFAULT, NL, true, true>
-                <<<(unsigned)(nwaves * (ny / NL::ROWS)), NL::ROW_THREADS, nsm, st>>>(a);
-        } else {
-            smem_attr(k_row_tt<N, L2_DEFAULT, L, true, true>, sm);
-            k_row_tt<N, L2_DEFAULT, L, true, true><<<grid, block, sm, st>>>(a);
-        }
-        return;
-    }
-    if (op == ROW_INV_T_FWD && (a.flags & PF_STORE_X)) op = ROW_INV_T_FWD_X;
-    else if (a.tt && op == ROW_INV_T_FWD) op = ROW_INV_TT_FWD;
-    else if (a.tt && op == ROW_T_FWD) op = ROW_TT_FWD;
     // the 12-warp form copies wave rows with 16-byte cp.async: it needs an aligned wave
-    if (op == ROW_INV_TT_FWD && a.variant == PASS_PIPELINED && ((uintptr_t)a.psi & 15) == 0 &&
-        row_q<N>(a, nwaves, ny, st))
+    if (op == ROW_INV_T_FWD && a.tt && !(a.flags & PF_STORE_X) && a.variant == PASS_PIPELINED &&
+        ((uintptr_t)a.psi & 15) == 0 && row_q<N>(a, nwaves, ny, st))
         return;
-    if (op == ROW_INV_TT_FWD && (a.tile & TILE_NARROW_ROWS)) {
-        // one warp of rows per block; only the transpose scratch lives in shared memory
-        using NL = NarrowLayout<N>;
-        auto kern = a.l2_mode == L2_WAVES_RESIDENT ? k_row_tt<N, L2_WAVES_RESIDENT, NL>
-                    : a.l2_mode == L2_SHARED_T     ? k_row_tt<N, L2_SHARED_T, NL>
-                                                   : k_row_tt<N, L2_DEFAULT, NL>;
-        const size_t nsm = sizeof(float2) * (size_t)NL::ROWS * NL::SCR_STRIDE_ROW;
+    using NL = NarrowLayout<N>;
+    const size_t sm = L::ROW_SMEM;
+    // one warp of rows per block: only the transpose scratch lives in shared memory
+    const size_t nsm = sizeof(float2) * (size_t)NL::ROWS * NL::SCR_STRIDE_ROW;
+    const bool narrow = (a.tile & TILE_NARROW_ROWS) != 0;
+    auto wide_step = [&](auto kern) {
+        smem_attr(kern, sm);
+        launch_step(kern, (unsigned)(nwaves * (ny / L::ROWS)), L::ROW_THREADS, sm, st, a.chained != 0, a);
+    };
+    auto narrow_step = [&](auto kern) {
         smem_attr(kern, nsm);
         launch_step(kern, (unsigned)(nwaves * (ny / NL::ROWS)), NL::ROW_THREADS, nsm, st, a.chained != 0, a);
+    };
+    if (op == ROW_INV_T_FWD && (a.flags & PF_STORE_X)) {
+        if (narrow && a.tt) narrow_step(k_row_tt<N, L2_DEFAULT, NL, false, ROWF_KEEP_X>);
+        else if (narrow) narrow_step(k_row_tt<N, L2_DEFAULT, NL, true, ROWF_KEEP_X>);
+        else if (a.tt) wide_step(k_row_tt<N, L2_DEFAULT, L, false, ROWF_KEEP_X>);
+        else wide_step(k_row_tt<N, L2_DEFAULT, L, true, ROWF_KEEP_X>);
+        return;
+    }
+    if (op == ROW_ADJ) {
+        if (narrow && a.tt) narrow_step(k_row_tt<N, L2_DEFAULT, NL, false, ROWF_ADJOINT>);
+        else if (narrow) narrow_step(k_row_tt<N, L2_DEFAULT, NL, true, ROWF_ADJOINT>);
+        else if (a.tt) wide_step(k_row_tt<N, L2_DEFAULT, L, false, ROWF_ADJOINT>);
+        else wide_step(k_row_tt<N, L2_DEFAULT, L, true, ROWF_ADJOINT>);
+        return;
+    }
+    if (op == ROW_INV_T_FWD && a.tt) {
+        if (narrow)
+            narrow_step(a.l2_mode == L2_WAVES_RESIDENT ? k_row_tt<N, L2_WAVES_RESIDENT, NL>
+                        : a.l2_mode == L2_SHARED_T     ? k_row_tt<N, L2_SHARED_T, NL>
+                                                       : k_row_tt<N, L2_DEFAULT, NL>);
+        else
+            wide_step(a.l2_mode == L2_WAVES_RESIDENT ? k_row_tt<N, L2_WAVES_RESIDENT>
+                      : a.l2_mode == L2_SHARED_T     ? k_row_tt<N, L2_SHARED_T>
+                                                     : k_row_tt<N, L2_DEFAULT>);
         return;
     }
     if (op == ROW_INV_T_FWD) {
-        // the row step on a σV store in the lean kernel (wide or narrow tiles; the wave stores keep
-        // the L2 mode's priority)
-        if (a.tile & TILE_NARROW_ROWS) {
-            using NL = NarrowLayout<N>;
-            auto kern = a.l2_mode == L2_WAVES_RESIDENT ? k_row_tt<N, L2_WAVES_RESIDENT, NL, true>
+        // the row step on a σV store
+        if (narrow)
+            narrow_step(a.l2_mode == L2_WAVES_RESIDENT ? k_row_tt<N, L2_WAVES_RESIDENT, NL, true>
                         : a.l2_mode == L2_SHARED_T     ? k_row_tt<N, L2_SHARED_T, NL, true>
-                                                       : k_row_tt<N, L2_DEFAULT, NL, true>;
-            const size_t nsm = sizeof(float2) * (size_t)NL::ROWS * NL::SCR_STRIDE_ROW;
-            smem_attr(kern, nsm);
-            launch_step(kern, (unsigned)(nwaves * (ny / NL::ROWS)), NL::ROW_THREADS, nsm, st, a.chained != 0, a);
-        } else {
-            auto kern = a.l2_mode == L2_WAVES_RESIDENT ? k_row_tt<N, L2_WAVES_RESIDENT, L, true>
-                        : a.l2_mode == L2_SHARED_T     ? k_row_tt<N, L2_SHARED_T, L, true>
-                                                       : k_row_tt<N, L2_DEFAULT, L, true>;
-            smem_attr(kern, sm);
-            launch_step(kern, grid.x, block.x, sm, st, a.chained != 0, a);
-        }
+                                                       : k_row_tt<N, L2_DEFAULT, NL, true>);
+        else
+            wide_step(a.l2_mode == L2_WAVES_RESIDENT ? k_row_tt<N, L2_WAVES_RESIDENT, L, true>
+                      : a.l2_mode == L2_SHARED_T     ? k_row_tt<N, L2_SHARED_T, L, true>
+                                                     : k_row_tt<N, L2_DEFAULT, L, true>);
         return;
     }
+    const dim3 grid((unsigned)(nwaves * (ny / L::ROWS))), block(L::ROW_THREADS);
+    auto other = [&](auto kern) {
+        smem_attr(kern, sm);
+        kern<<<grid, block, sm, st>>>(a);
+    };
     switch (op) {
     case ROW_T_FWD:
-        smem_attr(k_row<N, ROW_T_FWD>, sm);
-        k_row<N, ROW_T_FWD><<<grid, block, sm, st>>>(a);
+        if (a.tt) other(k_row<N, ROW_TT_FWD>);
+        else other(k_row<N, ROW_T_FWD>);
         break;
-    case ROW_INV_T_FWD:
-        smem_attr(k_row<N, ROW_INV_T_FWD>, sm);
-        k_row<N, ROW_INV_T_FWD><<<grid, block, sm, st>>>(a);
-        break;
-    case ROW_INV_ABS2:
-        smem_attr(k_row<N, ROW_INV_ABS2>, sm);
-        k_row<N, ROW_INV_ABS2><<<grid, block, sm, st>>>(a);
-        break;
-    case ROW_INV_STORE:
-        smem_attr(k_row<N, ROW_INV_STORE>, sm);
-        k_row<N, ROW_INV_STORE><<<grid, block, sm, st>>>(a);
-        break;
-    case ROW_ADJ:
-        smem_attr(k_row<N, ROW_ADJ>, sm);
-        k_row<N, ROW_ADJ><<<grid, block, sm, st>>>(a);
-        break;
-    case ROW_INV_T_FWD_X:
-        smem_attr(k_row<N, ROW_INV_T_FWD_X>, sm);
-        k_row<N, ROW_INV_T_FWD_X><<<grid, block, sm, st>>>(a);
-        break;
-    case ROW_INV_TT_FWD: {
-        auto kern = a.l2_mode == L2_WAVES_RESIDENT ? k_row_tt<N, L2_WAVES_RESIDENT>
-                                                   : (a.l2_mode == L2_SHARED_T ? k_row_tt<N, L2_SHARED_T>
-                                                                               : k_row_tt<N, L2_DEFAULT>);
-        smem_attr(kern, sm);
-        launch_step(kern, grid.x, block.x, sm, st, a.chained != 0, a);
-    } break;
-    case ROW_TT_FWD:
-        smem_attr(k_row<N, ROW_TT_FWD>, sm);
-        k_row<N, ROW_TT_FWD><<<grid, block, sm, st>>>(a);
-        break;
+    case ROW_INV_ABS2: other(k_row<N, ROW_INV_ABS2>); break;
+    case ROW_INV_STORE: other(k_row<N, ROW_INV_STORE>); break;
     default: throw MsError(MS_ERR_INTERNAL, "unknown row pass");
     }
 }
