@@ -20,6 +20,14 @@ struct ms_ctx {
     bool propT_built = false;                    // the table's transposed copy is current too
     void* exptab = nullptr;                      // exp(2 pi i k / 1024), k < 1024
     int* d_err = nullptr;                        // device word: a bounded device-side wait ran out
+    // Pinned host memory for a call's small uploads and read-backs (kStageBytes, taken front to back,
+    // free again when the call has ended): one page-locked copy is asynchronous, where each pageable
+    // copy costs the host and the GPU some microseconds.  The first bytes receive d_err.
+    char* stage = nullptr;
+    size_t stage_off = 0;
+    bool stage_busy = false;                     // a call is using it (or ended by an exception)
+    static constexpr size_t kStageBytes = 2u << 20, kStageFirst = 64;
+    void* stage_take(size_t bytes);              // null: no room, use the caller's memory
     int inject = 0;                              // host-side fault injection (MS_INJECT_*), for tests
 
     struct Buf {

@@ -67,6 +67,14 @@ void* ms_ctx::buf(const std::string& name, size_t bytes)
     return p;
 }
 
+void* ms_ctx::stage_take(size_t bytes)
+{
+    const size_t off = (stage_off + 63) / 64 * 64;
+    if (!stage || off + bytes > kStageBytes) return nullptr;
+    stage_off = off + bytes;
+    return stage + off;
+}
+
 void ms_ctx::drop_graph()
 {
     for (auto& kv : graphs)
@@ -88,6 +96,8 @@ void ms_ctx::release_all()
     exptab = nullptr;
     if (d_err) cudaFree(d_err);
     d_err = nullptr;
+    if (stage) cudaFreeHost(stage);
+    stage = nullptr;
     prop_key.clear();
 }
 
@@ -161,6 +171,16 @@ void run_potential(ms_ctx* c, const PotArgs& a, int n_conf, cudaStream_t st)
 
 namespace {
 constexpr double kPi = 3.14159265358979323846264338327950288;
+
+// Host memory to the device on `st`, through the call's pinned memory where it has room.
+void upload(ms_ctx* c, void* dst, const void* src, size_t bytes, cudaStream_t st)
+{
+    if (void* h = c->stage_take(bytes)) {
+        std::memcpy(h, src, bytes);
+        src = h;
+    }
+    CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
+}
 
 int team_size(int N)
 {
@@ -274,8 +294,6 @@ struct Setup {
     GridDev gd;
     const float2* tw_x;
     const float2* tw_y;
-    const float2* prop_x;
-    const float2* prop_y;
     const float2* prop;
     const float2* propT = nullptr;   // transposed propagator tables (1024-point columns), or null
     const float2* exptab;
@@ -308,24 +326,6 @@ Setup make_setup(ms_ctx* c, const ms_params& p)
     s.gd.g0y = s.gc.g0y;
     s.tw_x = twiddles(c, p.nx);
     s.tw_y = twiddles(c, p.ny);
-    // separable propagator phase exp(i w (g - g0)^2) per axis, formed in FP64 (device_kernels.cuh:215-234)
-    std::vector<float2> px(p.nx), py(p.ny);
-    for (int i = 0; i < p.nx; i++) {
-        double g = (double)((i < p.nx / 2) ? i : i - p.nx) * s.gc.dgx - s.gc.g0x;
-        double th = s.gc.prop_w * g * g;
-        px[i] = make_float2((float)std::cos(th), (float)std::sin(th));
-    }
-    for (int i = 0; i < p.ny; i++) {
-        double g = (double)((i < p.ny / 2) ? i : i - p.ny) * s.gc.dgy - s.gc.g0y;
-        double th = s.gc.prop_w * g * g;
-        py[i] = make_float2((float)std::cos(th), (float)std::sin(th));
-    }
-    float2* dpx = (float2*)c->buf("prop_x", sizeof(float2) * p.nx);
-    float2* dpy = (float2*)c->buf("prop_y", sizeof(float2) * p.ny);
-    CK(cudaMemcpyAsync(dpx, px.data(), sizeof(float2) * p.nx, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(dpy, py.data(), sizeof(float2) * p.ny, cudaMemcpyHostToDevice, c->stream));
-    s.prop_x = dpx;
-    s.prop_y = dpy;
     // full table P(k), rebuilt only when the grid, wavelength, slice thickness or tilt change
     char key[256];
     std::snprintf(key, sizeof(key), "%d,%d,%.17g,%.17g,%.17g,%.17g,%.17g,%d", p.nx, p.ny, p.lx, p.ly, s.gc.prop_w,
@@ -406,27 +406,36 @@ AtomsDev upload_atoms(ms_ctx* c, const ms_params& p, const ms_atoms& a)
         }
         tabs[i] = it->second;
     }
-    std::vector<int> el(a.n);
+    // everything in one device buffer and, when the call's pinned memory has room, one copy: the
+    // tables, the coefficients, then x, y, z, sigma, occupancy and element index of every atom
+    const size_t nt = sizeof(ElemTable) * tabs.size(), ncf = sizeof(ElemCoefDev) * zs.size();
+    const size_t row = (size_t)a.n * 4, head = (nt + ncf + 255) / 256 * 256, all = head + 6 * row;
+    char* dev = (char*)c->buf("atoms", all);
+    char* h = (char*)c->stage_take(all);
+    std::vector<char> own;   // the head and the element indexes, where the atoms' own arrays are copied
+    if (!h) own.resize(head + row);
+    char* hh = h ? h : own.data();
+    std::memcpy(hh, tabs.data(), nt);
+    for (size_t i = 0; i < zs.size(); i++) {
+        const ElemCoefDev cf = elem_coef_dev(p, zs[i]);
+        std::memcpy(hh + nt + i * sizeof(ElemCoefDev), &cf, sizeof(cf));
+    }
+    int* el = (int*)(hh + head + (h ? 5 * row : 0));
     for (int64_t i = 0; i < a.n; i++) el[i] = zmap[a.Z[i] & 127];
-    size_t fb = sizeof(float) * (size_t)a.n;
-    float* x = (float*)c->buf("at_x", fb);
-    float* y = (float*)c->buf("at_y", fb);
-    float* z = (float*)c->buf("at_z", fb);
-    float* sg = (float*)c->buf("at_s", fb);
-    float* oc = (float*)c->buf("at_o", fb);
-    int* e = (int*)c->buf("at_e", sizeof(int) * (size_t)a.n);
-    ElemTable* t = (ElemTable*)c->buf("at_tab", sizeof(ElemTable) * tabs.size());
-    CK(cudaMemcpyAsync(x, a.x, fb, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(y, a.y, fb, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(z, a.z, fb, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(sg, a.sigma, fb, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(oc, a.occ, fb, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(e, el.data(), sizeof(int) * (size_t)a.n, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(t, tabs.data(), sizeof(ElemTable) * tabs.size(), cudaMemcpyHostToDevice, c->stream));
-    std::vector<ElemCoefDev> cf(zs.size());
-    for (size_t i = 0; i < zs.size(); i++) cf[i] = elem_coef_dev(p, zs[i]);
-    ElemCoefDev* dcf = (ElemCoefDev*)c->buf("at_coef", sizeof(ElemCoefDev) * cf.size());
-    CK(cudaMemcpyAsync(dcf, cf.data(), sizeof(ElemCoefDev) * cf.size(), cudaMemcpyHostToDevice, c->stream));
+    const float* arr[5] = {a.x, a.y, a.z, a.sigma, a.occ};
+    if (h) {
+        for (int k = 0; k < 5; k++) std::memcpy(h + head + k * row, arr[k], row);
+        CK(cudaMemcpyAsync(dev, h, all, cudaMemcpyHostToDevice, c->stream));
+    } else {
+        CK(cudaMemcpyAsync(dev, hh, head, cudaMemcpyHostToDevice, c->stream));
+        for (int k = 0; k < 5; k++)
+            CK(cudaMemcpyAsync(dev + head + k * row, arr[k], row, cudaMemcpyHostToDevice, c->stream));
+        CK(cudaMemcpyAsync(dev + head + 5 * row, el, row, cudaMemcpyHostToDevice, c->stream));
+    }
+    const ElemTable* t = (const ElemTable*)dev;
+    const ElemCoefDev* dcf = (const ElemCoefDev*)(dev + nt);
+    const float *x = (const float*)(dev + head), *y = x + a.n, *z = y + a.n, *sg = z + a.n, *oc = sg + a.n;
+    const int* e = (const int*)(oc + a.n);
     d.coefs = dcf;
     d.x = x; d.y = y; d.z = z; d.sig = sg; d.occ = oc; d.elem = e; d.tables = t;
     d.n_elem = (int)tabs.size();
@@ -467,18 +476,23 @@ SpecGroup build_specimen(ms_ctx* c, const ms_params& p, const AtomsDev& A, const
     const int64_t n = A.n, nc = g.nconf;
     cudaStream_t st = c->stream;
     int* dconf = (int*)c->buf("sp_conf", sizeof(int) * nc);
-    CK(cudaMemcpyAsync(dconf, confs.data(), sizeof(int) * nc, cudaMemcpyHostToDevice, st));
+    upload(c, dconf, confs.data(), sizeof(int) * nc, st);
     size_t fb = sizeof(float) * (size_t)(n * nc);
     float* xd = (float*)c->buf("sp_xd", fb);
     float* yd = (float*)c->buf("sp_yd", fb);
     float* zd = (float*)c->buf("sp_zd", fb);
-    launch_displace(A.x, A.y, A.z, A.sig, n, dconf, (int)nc, p.pn_seed, p.pn_dim_x, p.pn_dim_y, p.pn_dim_z, xd, yd,
-                    zd, st);
     unsigned* zr = (unsigned*)c->buf("sp_zr", sizeof(unsigned) * 2 * nc);
-    launch_zrange(zd, n, (int)nc, zr, zr + nc, st);
-    std::vector<unsigned> zh(2 * nc);
-    CK(cudaMemcpyAsync(zh.data(), zr, sizeof(unsigned) * 2 * nc, cudaMemcpyDeviceToHost, st));
+    launch_displace(A.x, A.y, A.z, A.sig, n, dconf, (int)nc, p.pn_seed, p.pn_dim_x, p.pn_dim_y, p.pn_dim_z, xd, yd,
+                    zd, zr, st);
+    std::vector<unsigned> zown;
+    unsigned* zh = (unsigned*)c->stage_take(sizeof(unsigned) * 2 * nc);
+    if (!zh) {
+        zown.resize(2 * nc);
+        zh = zown.data();
+    }
+    CK(cudaMemcpyAsync(zh, zr, sizeof(unsigned) * 2 * nc, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    for (int i = 0; i < nc; i++) zh[i] = ~zh[i];   // the minimum is kept complemented
     // slicing planes on the host, bit-identical with the device arithmetic
     const float dz = (float)p.dz;
     const int border = border_of(p);
@@ -510,14 +524,18 @@ SpecGroup build_specimen(ms_ctx* c, const ms_params& p, const AtomsDev& A, const
         g.z_init[i] = (double)(float)(0.5 * (double)sum);  // Slice::z_m (slice.hpp:19-22)
     }
     g.S_cap = S_cap;
-    float* db = (float*)c->buf("sp_bounds", sizeof(float) * bounds.size());
-    int* dnv = (int*)c->buf("sp_nv", sizeof(int) * nc);
-    float* dvmax = (float*)c->buf("sp_vmax", sizeof(float) * nc);
-    int* dns = (int*)c->buf("sp_ns", sizeof(int) * nc);
-    CK(cudaMemcpyAsync(db, bounds.data(), sizeof(float) * bounds.size(), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(dnv, nv.data(), sizeof(int) * nc, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(dvmax, vmax.data(), sizeof(float) * nc, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(dns, g.ns.data(), sizeof(int) * nc, cudaMemcpyHostToDevice, st));
+    // planes, plane counts, highest atoms and slice counts in one copy
+    const size_t nb = bounds.size();
+    std::vector<float> planes(nb + 3 * (size_t)nc);
+    std::copy(bounds.begin(), bounds.end(), planes.begin());
+    std::memcpy(planes.data() + nb, nv.data(), 4 * (size_t)nc);
+    std::memcpy(planes.data() + nb + nc, vmax.data(), 4 * (size_t)nc);
+    std::memcpy(planes.data() + nb + 2 * nc, g.ns.data(), 4 * (size_t)nc);
+    float* db = (float*)c->buf("sp_planes", sizeof(float) * planes.size());
+    upload(c, db, planes.data(), sizeof(float) * planes.size(), st);
+    const int* dnv = (const int*)(db + nb);
+    const float* dvmax = db + nb + nc;
+    const int* dns = (const int*)(db + nb + 2 * nc);
     // spatial cells: at least the largest cut-off and a quarter of a potential tile (64 x 32 pixels),
     // so a tile touches at most 7 x 5 cells
     const double cell = std::max({(double)A.rmax_all, 16.0 * p.lx / p.nx, 16.0 * p.ly / p.ny, 0.25});
@@ -691,8 +709,6 @@ PassArgs pass_args(const Setup& s, float2* psi, const WaveInfo* waves, const flo
     a.sV = sV;
     a.sV_slot_stride = slot_stride;
     a.sV_slice_base = 0;
-    a.prop_x = s.prop_x;
-    a.prop_y = s.prop_y;
     a.prop = s.prop;
     a.propT = s.propT;
     a.exptab = s.exptab;
@@ -862,8 +878,7 @@ EngineArgs engine_plan(ms_ctx* c, const std::vector<int>& ns, int slice0, int N,
     unsigned* cnt = (unsigned*)c->buf("eng_cnt" + tag, sizeof(unsigned) * 2 * nw);
     CK(cudaMemsetAsync(e.state, 0, sizeof(EngineState), st));
     CK(cudaMemsetAsync(cnt, 0, sizeof(unsigned) * 2 * nw, st));
-    // pageable source: the copy has read the table when the call returns
-    CK(cudaMemcpyAsync(dstart, start.data(), sizeof(int) * start.size(), cudaMemcpyHostToDevice, st));
+    upload(c, dstart, start.data(), sizeof(int) * start.size(), st);
     e.phase_start = dstart;
     e.n_items = t;
     e.S_max = S;
@@ -902,15 +917,22 @@ struct Timer {
     int64_t l0;
     explicit Timer(ms_ctx* cc) : c(cc), l0(kernel_launches())
     {
+        // a call that ended by an exception may have left copies from the pinned memory in flight
+        if (c->stage_busy) CK(cudaDeviceSynchronize());
+        c->stage_off = ms_ctx::kStageFirst;
+        c->stage_busy = true;
         CK(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
         CK(cudaEventRecord(c->ev0, c->stream));
     }
     void stop()
     {
         CK(cudaEventRecord(c->ev1, c->stream));
-        CK(cudaEventSynchronize(c->ev1));
-        int e = 0;
-        CK(cudaMemcpy(&e, c->d_err, sizeof(int), cudaMemcpyDeviceToHost));
+        int pageable = 0;
+        int* h = c->stage ? (int*)c->stage : &pageable;
+        CK(cudaMemcpyAsync(h, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+        c->stage_busy = false;
+        const int e = *h;
         if (e & 1) throw MsError(MS_ERR_TIMEOUT, "a device-side wait for a shared-memory tile ran out");
         if (e) throw MsError(MS_ERR_TIMEOUT, "a device-side wait for another block's slice work ran out");
         float ms = 0.f;
@@ -962,6 +984,10 @@ void ctx_activate(ms_ctx* c)
         CK(cudaMalloc(&c->d_err, sizeof(int)));
         c->forget_free_mem();
         CK(cudaMemset(c->d_err, 0, sizeof(int)));
+    }
+    if (!c->stage && cudaMallocHost((void**)&c->stage, ms_ctx::kStageBytes) != cudaSuccess) {
+        cudaGetLastError();   // without it the copies are pageable
+        c->stage = nullptr;
     }
 }
 
@@ -1096,7 +1122,7 @@ void sim_tem_like(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* o
             wv[i].pos = 0;
         }
         WaveInfo* dwv = (WaveInfo*)c->buf("waves", sizeof(WaveInfo) * nw);
-        CK(cudaMemcpyAsync(dwv, wv.data(), sizeof(WaveInfo) * nw, cudaMemcpyHostToDevice, st));
+        upload(c, dwv, wv.data(), sizeof(WaveInfo) * nw, st);
         float2* psi = (float2*)c->buf("psi", sizeof(float2) * N * nw);
         PassArgs pa = pass_args(s, psi, dwv, sVs, slot, cond);
         pa.l2_mode = l2_mode_for_waves(nw, N);
@@ -1262,7 +1288,6 @@ void sim_tem_like(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* o
             else launch_acc_abs2(psi, nw, dwv, N, acc, first, st);
         }
         first = false;
-        CK(cudaStreamSynchronize(st));  // host wave table reused by the next group
     }
     float* o0 = (float*)c->buf("out0", sizeof(float) * N * nimg);
     for (int i = 0; i < nimg; i++) launch_emit(acc + (size_t)i * N, p.nx, p.ny, kspace ? 1 : 0, o0 + (size_t)i * N, st);
@@ -1359,6 +1384,29 @@ int autotune_batch(ms_ctx* c, const ms_params& p, const Setup& s, const PassArgs
 }
 
 }  // namespace
+
+// Pixels inside the probe's aperture: det_g2 (the sum of the two axes' squared float frequencies)
+// against the thresholds, with each axis squared once.
+static double aperture_pixels(const ms_params& p, const GridConst& gc, const LensCoef& L)
+{
+    std::vector<float> gx2(p.nx);
+    for (int ix = 0; ix < p.nx; ix++) {
+        const float g = det_gfreq(ix, p.nx, gc.dgx_f);
+        gx2[ix] = MSF_MUL(g, g);
+    }
+    int64_t n = 0;
+    for (int iy = 0; iy < p.ny; iy++) {
+        const float g = det_gfreq(iy, p.ny, gc.dgy_f), gy2 = MSF_MUL(g, g);
+        if (gy2 >= L.g2max) continue;   // no column brings it back below
+        int row = 0;
+        for (int ix = 0; ix < p.nx; ix++) {
+            const float g2 = MSF_ADD(gx2[ix], gy2);
+            row += (L.g2min <= g2) & (g2 < L.g2max);
+        }
+        n += row;
+    }
+    return (double)n;
+}
 
 // General scan (run_STEM_general_simu, scan_simulator.cuh:115-183): for every phonon configuration
 // and probe position, the grid box is a window of lx x ly centred on the probe; the displaced atoms
@@ -1472,17 +1520,7 @@ void sim_stem_general(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_outpu
     out->interval_x = p.scan_dx;
     out->interval_y = p.scan_dy;
     out->n_slices = 0;
-    double tot = 0.0;
-    {
-        const GridConst gc = grid_of(p, ph);
-        const LensCoef L = lens_coef(p.cond_lens, ph.lambda, 0.0);
-        for (int iy = 0; iy < p.ny; iy++)
-            for (int ix = 0; ix < p.nx; ix++) {
-                const float g2 = det_g2(ix, iy, p.nx, p.ny, gc.dgx_f, gc.dgy_f);
-                if (L.g2min <= g2 && g2 < L.g2max) tot += 1.0;
-            }
-    }
-    out->total_intensity = tot * (double)N * (double)N;
+    out->total_intensity = aperture_pixels(p, grid_of(p, ph), lens_coef(p.cond_lens, ph.lambda, 0.0)) * (double)N * (double)N;
 }
 
 void sim_stem(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* out)
@@ -1511,7 +1549,7 @@ void sim_stem(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* out)
         thr[ndet + d] = g2_threshold(p.det_outer[d], s.ph.lambda);
     }
     float* dthr = (float*)c->buf("det_thr", sizeof(float) * 2 * ndet);
-    CK(cudaMemcpyAsync(dthr, thr.data(), sizeof(float) * 2 * ndet, cudaMemcpyHostToDevice, st));
+    upload(c, dthr, thr.data(), sizeof(float) * 2 * ndet, st);
     double* img = (double*)c->buf("stem_acc", sizeof(double) * ndet * npos);
     CK(cudaMemsetAsync(img, 0, sizeof(double) * ndet * npos, st));
     const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>(64, N / 4096));
@@ -1550,7 +1588,7 @@ void sim_stem(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* out)
             wv[ip].pos = ip;
         }
         WaveInfo* dwv_all = (WaveInfo*)c->buf("waves_all", sizeof(WaveInfo) * npos);
-        CK(cudaMemcpyAsync(dwv_all, wv.data(), sizeof(WaveInfo) * npos, cudaMemcpyHostToDevice, st));
+        upload(c, dwv_all, wv.data(), sizeof(WaveInfo) * npos, st);
         if (!tuned) {
             PassArgs base = pass_args(s, nullptr, nullptr, nullptr, slot, cond);
             base.tt = sT;
@@ -1631,16 +1669,7 @@ void sim_stem(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* out)
     out->n_slices = 0;
     // total_intensity: vacuum exit intensity sum_k N^2 A(k) (the reference's blank intensity
     // table, scan_simulator.cuh:34); probes have |Psi0(k)| in {0,1}
-    {
-        LensCoef L = lens_coef(p.cond_lens, s.ph.lambda, 0.0);
-        double tot = 0.0;
-        for (int iy = 0; iy < p.ny; iy++)
-            for (int ix = 0; ix < p.nx; ix++) {
-                float g2 = det_g2(ix, iy, p.nx, p.ny, s.gd.dgx_f, s.gd.dgy_f);
-                if (L.g2min <= g2 && g2 < L.g2max) tot += 1.0;
-            }
-        out->total_intensity = tot * (double)N * (double)N;
-    }
+    out->total_intensity = aperture_pixels(p, s.gc, lens_coef(p.cond_lens, s.ph.lambda, 0.0)) * (double)N * (double)N;
 }
 
 // ---------------------------------------------------------------------------
@@ -1699,7 +1728,7 @@ void sim_thickness(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* 
             wv[i].n_slices = g.ns[i];
         }
         WaveInfo* dwv = (WaveInfo*)c->buf("waves", sizeof(WaveInfo) * wv.size());
-        CK(cudaMemcpyAsync(dwv, wv.data(), sizeof(WaveInfo) * wv.size(), cudaMemcpyHostToDevice, st));
+        upload(c, dwv, wv.data(), sizeof(WaveInfo) * wv.size(), st);
         float2* psi = (float2*)c->buf("psi", sizeof(float2) * N * nw);
         float2* aux = (float2*)c->buf("thick_aux", sizeof(float2) * N * nw * chunk);
         PassArgs pa = pass_args(s, psi, dwv, nullptr, slot, cond);
@@ -1750,7 +1779,6 @@ void sim_thickness(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* 
             }
         };
         run_graphed(c, graph_key_of(pa, nw, nf, iw, chunk, aux, frames, nullptr, nullptr, -2), slices);
-        CK(cudaStreamSynchronize(st));  // the host wave table is reused by the next group
     }
     copy_out(c, out->thickness_frames, frames, (int64_t)nf * N, out->on_device);
     tm.stop();
@@ -1781,9 +1809,10 @@ void sim_potential(ms_ctx* c, const ms_params& p, const ms_atoms& a, int conf, f
     if (V) {
         MS_REQUIRE((int64_t)S * s.N <= cap, MS_ERR_INVALID_ARG, "V_out holds fewer than n_slices*ny*nx floats");
         int64_t slot = (int64_t)S * s.N;
-        float* sV = (float*)c->buf("sV", sizeof(float) * slot);
+        // straight into a device buffer of the caller's (the kernel stores single floats)
+        float* sV = on_dev ? V : (float*)c->buf("sV", sizeof(float) * slot);
         run_potential(c, pot_args(p, s, A, g, sV, slot, 0, S, 0), 1, st);
-        copy_out(c, V, sV, slot, on_dev);
+        if (!on_dev) copy_out(c, V, sV, slot, 0);
     }
     tm.stop();
 }
@@ -1829,7 +1858,7 @@ void sim_stem_forward_potential(ms_ctx* c, const ms_params& p, const float* V, i
         thr[ndet + d] = g2_threshold(p.det_outer[d], s.ph.lambda);
     }
     float* dthr = (float*)c->buf("det_thr", sizeof(float) * 2 * ndet);
-    CK(cudaMemcpyAsync(dthr, thr.data(), sizeof(float) * 2 * ndet, cudaMemcpyHostToDevice, st));
+    upload(c, dthr, thr.data(), sizeof(float) * 2 * ndet, st);
     float2* sT = caller_transmission(c, s, sV, slot, np);
     const int B = std::min(np, p.probe_batch > 0 ? p.probe_batch : 256);
     const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>(64, N / 4096));
@@ -1849,7 +1878,7 @@ void sim_stem_forward_potential(ms_ctx* c, const ms_params& p, const float* V, i
             wv[i].pos = start + i;
         }
         WaveInfo* dwv = (WaveInfo*)c->buf("waves", sizeof(WaveInfo) * B);
-        CK(cudaMemcpyAsync(dwv, wv.data(), sizeof(WaveInfo) * nb, cudaMemcpyHostToDevice, st));
+        upload(c, dwv, wv.data(), sizeof(WaveInfo) * nb, st);
         float2* psi = (float2*)c->buf("psi", sizeof(float2) * N * B);
         PassArgs pa = pass_args(s, psi, dwv, sV, slot, cond);
         pa.tt = sT;
@@ -1912,9 +1941,9 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
         thr[ndet + d] = g2_threshold(p.det_outer[d], s.ph.lambda);
     }
     float* dthr = (float*)c->buf("det_thr", sizeof(float) * 2 * ndet);
-    CK(cudaMemcpyAsync(dthr, thr.data(), sizeof(float) * 2 * ndet, cudaMemcpyHostToDevice, st));
+    upload(c, dthr, thr.data(), sizeof(float) * 2 * ndet, st);
     float* dtgt = (float*)c->buf("adj_target", sizeof(float) * np * ndet);
-    CK(cudaMemcpyAsync(dtgt, target, sizeof(float) * np * ndet, cudaMemcpyHostToDevice, st));
+    upload(c, dtgt, target, sizeof(float) * np * ndet, st);
 
     float2* sT = caller_transmission(c, s, sV, slot, np);
     const int k = p.ckpt_interval;
@@ -1956,7 +1985,7 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
             wv[i].pos = start + i;
         }
         WaveInfo* dwv = (WaveInfo*)c->buf("waves", sizeof(WaveInfo) * B);
-        CK(cudaMemcpyAsync(dwv, wv.data(), sizeof(WaveInfo) * nb, cudaMemcpyHostToDevice, st));
+        upload(c, dwv, wv.data(), sizeof(WaveInfo) * nb, st);
         PassArgs pa = pass_args(s, adj, dwv, sV, slot, cond);
         pa.tt = sT;
         pa.l2_mode = l2_mode_for_waves(nb, N);
@@ -2143,7 +2172,8 @@ void sim_many(ms_ctx* c, int n, const ms_params* ps, const ms_atoms* as, ms_outp
     for (int i = 0; i < n; i++) {
         const int64_t N = (int64_t)ps[i].nx * ps[i].ny;
         const ConfSet cs = conf_set(ps[i]);
-        need[i] = (size_t)N * (4 * (size_t)estimate_slices(ps[i], as[i]) * cs.confs.size() + 8 + 4 + 8 * cs.confs.size());
+        need[i] = (size_t)N * (4 * (size_t)estimate_slices(ps[i], as[i]) * cs.confs.size() + 8 * kPropSets + 4 +
+                               8 * cs.confs.size()) + 4 * 256;
     }
     int r0 = 0;
     while (r0 < n) {
@@ -2273,7 +2303,7 @@ void sim_many(ms_ctx* c, int n, const ms_params* ps, const ms_atoms* as, ms_outp
             G.acc = (double*)c->buf("many_acc_" + tag, sizeof(double) * N);
             G.s = side_stream(c, gi);
             CK(cudaStreamWaitEvent(G.s, fork, 0));
-            CK(cudaMemcpyAsync(G.dwv, G.waves.data(), sizeof(WaveInfo) * G.waves.size(), cudaMemcpyHostToDevice, G.s));
+            upload(c, G.dwv, G.waves.data(), sizeof(WaveInfo) * G.waves.size(), G.s);
         }
         // probes, per instance (each has its own lens, grid and wavelength)
         for (Group& G : groups) {

@@ -407,6 +407,7 @@ void validate_params(const ms_params& p)
     MS_REQUIRE(p.probe_batch >= 0 && p.probe_batch <= 4096, MS_ERR_INVALID_ARG, "probe_batch out of range");
 }
 
+__attribute__((optimize("O3")))   // vectorised: these passes are most of a small call's checks
 void validate_atoms(const ms_params& p, const ms_atoms* a)
 {
     (void)p;
@@ -414,12 +415,17 @@ void validate_atoms(const ms_params& p, const ms_atoms* a)
     MS_REQUIRE(a->n >= 1, MS_ERR_INVALID_ARG, "the specimen has no atoms");
     MS_REQUIRE(a->n <= (1LL << 31) - 1, MS_ERR_INVALID_ARG, "too many atoms");
     MS_REQUIRE(a->Z && a->x && a->y && a->z && a->sigma && a->occ, MS_ERR_INVALID_ARG, "atom arrays must not be NULL");
-    for (int64_t i = 0; i < a->n; i++) {
-        MS_REQUIRE(a->Z[i] >= 1 && a->Z[i] <= 103, MS_ERR_INVALID_ARG, "atomic number out of range");
-        MS_REQUIRE(std::isfinite(a->x[i]) && std::isfinite(a->y[i]) && std::isfinite(a->z[i]) &&
-                       std::isfinite(a->sigma[i]) && std::isfinite(a->occ[i]),
-                   MS_ERR_INVALID_ARG, "atom coordinates must be finite");
-    }
+    // branch-free passes over the arrays (exponent bits all set: infinite or not a number)
+    unsigned bad_z = 0, bad = 0;
+    for (int64_t i = 0; i < a->n; i++) bad_z |= (unsigned)(a->Z[i] - 1) > 102u;
+    for (const float* f : {a->x, a->y, a->z, a->sigma, a->occ})
+        for (int64_t i = 0; i < a->n; i++) {
+            uint32_t u;
+            std::memcpy(&u, f + i, 4);
+            bad |= (u & 0x7f800000u) == 0x7f800000u;
+        }
+    MS_REQUIRE(!bad_z, MS_ERR_INVALID_ARG, "atomic number out of range");
+    MS_REQUIRE(!bad, MS_ERR_INVALID_ARG, "atom coordinates must be finite");
 }
 
 }  // namespace msb

@@ -668,63 +668,48 @@ void launch_potential(const PotArgs& a, int n_conf, cudaStream_t st)
 // ---------------------------------------------------------------------------
 // specimen on the device: displacement, z range, slice assignment, gather
 // ---------------------------------------------------------------------------
-__global__ void k_displace(const float* x, const float* y, const float* z, const float* sig, int64_t n,
-                           const int* confs, uint64_t seed, int dx, int dy, int dzf, float* xd, float* yd, float* zd)
-{
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int ci = blockIdx.y;
-    float xi = x[i], yi = y[i], zi = z[i];
-    det_displace(seed, confs[ci], i, sig[i], dx, dy, dzf, &xi, &yi, &zi);
-    int64_t o = (int64_t)ci * n + i;
-    xd[o] = xi;
-    yd[o] = yi;
-    zd[o] = zi;
-}
-
-void launch_displace(const float* x, const float* y, const float* z, const float* sig, int64_t n, const int* confs,
-                     int nconf, uint64_t seed, int dx, int dy, int dzf, float* xd, float* yd, float* zd,
-                     cudaStream_t st)
-{
-    dim3 grid((unsigned)((n + 255) / 256), (unsigned)nconf);
-    k_displace<<<grid, 256, 0, st>>>(x, y, z, sig, n, confs, seed, dx, dy, dzf, xd, yd, zd);
-    count_launch();
-    check_launch("displace");
-}
-
 __device__ __forceinline__ unsigned f2ord(float f)
 {
     unsigned b = __float_as_uint(f);
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 
-__global__ void k_zrange(const float* zd, int64_t n, unsigned* zmin, unsigned* zmax)
+// Displaced atoms of every configuration, and each configuration's z range in zrange (order-preserving
+// keys; [nconf] complemented minima, then [nconf] maxima, both reduced as maxima from zero).
+__global__ void k_displace(const float* x, const float* y, const float* z, const float* sig, int64_t n,
+                           const int* confs, uint64_t seed, int dx, int dy, int dzf, float* xd, float* yd, float* zd,
+                           unsigned* zrange)
 {
-    int ci = blockIdx.y;
-    unsigned lo = 0xFFFFFFFFu, hi = 0u;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        unsigned k = f2ord(zd[(int64_t)ci * n + i]);
-        lo = min(lo, k);
-        hi = max(hi, k);
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int ci = blockIdx.y;
+    unsigned lo = 0u, hi = 0u;
+    if (i < n) {
+        float xi = x[i], yi = y[i], zi = z[i];
+        det_displace(seed, confs[ci], i, sig[i], dx, dy, dzf, &xi, &yi, &zi);
+        const int64_t o = (int64_t)ci * n + i;
+        xd[o] = xi;
+        yd[o] = yi;
+        zd[o] = zi;
+        hi = f2ord(zi);
+        lo = ~hi;
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    }
+    lo = __reduce_max_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
     if ((threadIdx.x & 31) == 0) {
-        atomicMin(zmin + ci, lo);
-        atomicMax(zmax + ci, hi);
+        atomicMax(zrange + ci, lo);
+        atomicMax(zrange + gridDim.y + ci, hi);
     }
 }
 
-void launch_zrange(const float* zd, int64_t n, int nconf, unsigned* zmin_bits, unsigned* zmax_bits, cudaStream_t st)
+void launch_displace(const float* x, const float* y, const float* z, const float* sig, int64_t n, const int* confs,
+                     int nconf, uint64_t seed, int dx, int dy, int dzf, float* xd, float* yd, float* zd,
+                     unsigned* zrange, cudaStream_t st)
 {
-    cudaMemsetAsync(zmin_bits, 0xFF, sizeof(unsigned) * nconf, st);
-    cudaMemsetAsync(zmax_bits, 0x00, sizeof(unsigned) * nconf, st);
-    int blocks = (int)std::min<int64_t>(1184, (n + 255) / 256);
-    k_zrange<<<dim3(blocks, nconf), 256, 0, st>>>(zd, n, zmin_bits, zmax_bits);
+    cudaMemsetAsync(zrange, 0, sizeof(unsigned) * 2 * nconf, st);
+    dim3 grid((unsigned)((n + 255) / 256), (unsigned)nconf);
+    k_displace<<<grid, 256, 0, st>>>(x, y, z, sig, n, confs, seed, dx, dy, dzf, xd, yd, zd, zrange);
     count_launch();
-    check_launch("z range");
+    check_launch("displace");
 }
 
 // Periodic wrap count of a coordinate (0 without wrapping), clamped to the 4 bits it is packed in.

@@ -211,8 +211,7 @@ void launch_prop_table(int nx, int ny, double dgx, double dgy, double g0x, doubl
 // specimen on the device
 void launch_displace(const float* x, const float* y, const float* z, const float* sig, int64_t n, const int* confs,
                      int nconf, uint64_t seed, int dx, int dy, int dzf, float* xd, float* yd, float* zd,
-                     cudaStream_t st);
-void launch_zrange(const float* zd, int64_t n, int nconf, unsigned* zmin_bits, unsigned* zmax_bits, cudaStream_t st);
+                     unsigned* zrange, cudaStream_t st);
 void launch_assign(const float* xd, const float* yd, const float* zd, int64_t n, int nconf, const float* bounds,
                    int bstride, const int* nv, const float* vmax, int S_cap, const CellGrid& cg, unsigned* keys,
                    int* vals, unsigned* counts, cudaStream_t st);

@@ -96,11 +96,11 @@ __global__ void __launch_bounds__(FftLayout<N>::ROW_THREADS, FftLayout<N>::ROW_M
         team_fft<N, G, -1>(v, g, tw, scr, sync);
 #pragma unroll
         for (int j = 0; j < E; j++) a.psi[row_off + g + G * j] = v[j];
-        return;
-    }
+    } else {
 #pragma unroll
-    for (int j = 0; j < E; j++) v[j] = a.psi[row_off + g + G * j];
-    team_fft<N, G, +1>(v, g, tw, scr, sync);
+        for (int j = 0; j < E; j++) v[j] = a.psi[row_off + g + G * j];
+        team_fft<N, G, +1>(v, g, tw, scr, sync);
+    }
     if constexpr (OP == ROW_INV_ABS2) {
         float* o = a.out_real + row_off;
         const float w = wi.weight;
