@@ -196,11 +196,12 @@ int team_size(int N)
 
 // Inter-level twiddles W_N^(g k1) at [k1 * G + g], in kTwSets dithered sets of N entries (set t
 // used by the slices s with s mod kTwSets = t), from FP64 values.
-const float2* twiddles(ms_ctx* c, int N)
+const float2* twiddles(ms_ctx* c, int N, int team = 0)
 {
-    auto it = c->twiddles.find(N);
+    const int key = team ? -N : N;   // the 64-thread teams' tables beside the usual ones
+    auto it = c->twiddles.find(key);
     if (it != c->twiddles.end()) return (const float2*)it->second;
-    int G = team_size(N), E = N / G;
+    int G = team ? team : team_size(N), E = N / G;
     std::vector<float2> t((size_t)kTwSets * N);
     for (int k1 = 0; k1 < E; k1++)
         for (int g = 0; g < G; g++) {
@@ -211,8 +212,14 @@ const float2* twiddles(ms_ctx* c, int N)
     CK(cudaMalloc(&p, sizeof(float2) * t.size()));
     c->forget_free_mem();
     CK(cudaMemcpy(p, t.data(), sizeof(float2) * t.size(), cudaMemcpyHostToDevice));
-    c->twiddles[N] = p;
+    c->twiddles[key] = p;
     return (const float2*)p;
+}
+
+// the tables of the 2048-point steps on 64-thread teams, where an axis has that length
+const float2* twiddles64(ms_ctx* c, int nx, int ny)
+{
+    return nx == 2048 || ny == 2048 ? twiddles(c, 2048, 64) : nullptr;
 }
 
 LensDev lens_dev(const LensCoef& L)
@@ -294,6 +301,7 @@ struct Setup {
     GridDev gd;
     const float2* tw_x;
     const float2* tw_y;
+    const float2* tw64;
     const float2* prop;
     const float2* propT = nullptr;   // transposed propagator tables (1024-point columns), or null
     const float2* exptab;
@@ -326,6 +334,7 @@ Setup make_setup(ms_ctx* c, const ms_params& p)
     s.gd.g0y = s.gc.g0y;
     s.tw_x = twiddles(c, p.nx);
     s.tw_y = twiddles(c, p.ny);
+    s.tw64 = twiddles64(c, p.nx, p.ny);
     // full table P(k), rebuilt only when the grid, wavelength, slice thickness or tilt change
     char key[256];
     std::snprintf(key, sizeof(key), "%d,%d,%.17g,%.17g,%.17g,%.17g,%.17g,%d", p.nx, p.ny, p.lx, p.ly, s.gc.prop_w,
@@ -711,6 +720,7 @@ PassArgs pass_args(const Setup& s, float2* psi, const WaveInfo* waves, const flo
     a.sV_slice_base = 0;
     a.prop = s.prop;
     a.propT = s.propT;
+    a.tw64 = s.tw64;
     a.exptab = s.exptab;
     a.grid = s.gd;
     a.lens = lens;
@@ -896,7 +906,8 @@ EngineArgs engine_plan(ms_ctx* c, const std::vector<int>& ns, int slice0, int N,
 // otherwise the batch runs slice by slice.
 bool engine_fits(const ms_ctx* c, int nx, int ny, int flags, bool uneven = false)
 {
-    const bool wanted = c->pass_variant == PASS_ENGINE || (uneven && c->pass_variant == PASS_CLASSIC);
+    // (2048-point groups of an uneven batch: the per-slice steps on 64-thread teams are faster)
+    const bool wanted = c->pass_variant == PASS_ENGINE || (uneven && c->pass_variant == PASS_CLASSIC && nx < 2048);
     return wanted && nx == ny && tensor_maps_available() &&
            !(flags & (PF_STORE_X | PF_FILTER_AUX | PF_VACUUM_BEYOND | PF_PROP_ALWAYS | PF_TILT_INCIDENT));
 }
@@ -1992,6 +2003,7 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
         upload(c, dwv, wv.data(), sizeof(WaveInfo) * nb, st);
         PassArgs pa = pass_args(s, adj, dwv, sV, slot, cond);
         pa.tt = sT;
+        pa.tw64 = nullptr;   // the adjoint's row and column steps are those of the 32-thread teams
         pa.l2_mode = l2_mode_for_waves(nb, N);
         pa.tile = choose_tile(c, pa, p.nx, p.ny, nb, S, st);
         pa.det_thr = dthr;
@@ -2284,6 +2296,7 @@ void sim_many(ms_ctx* c, int n, const ms_params* ps, const ms_atoms* as, ms_outp
         for (Group& G : groups) {
             twiddles(c, G.nx);
             twiddles(c, G.ny);
+            twiddles64(c, G.nx, G.ny);
             G.done_off = nwaves_all;
             for (int i : G.inst) nwaves_all += in[i].waves.size();
             G.engine = engine_fits(c, G.nx, G.ny, 0, true);
@@ -2366,6 +2379,8 @@ void sim_many(ms_ctx* c, int n, const ms_params* ps, const ms_atoms* as, ms_outp
                 pa.exptab = ex;
                 pa.grid = in[G.inst.front()].gd;
                 pa.err = c->d_err;
+                pa.tile = TILE_NARROW_ROWS;   // the faster row step at every length on batches
+                pa.tw64 = twiddles64(c, G.nx, G.ny);
                 pa.tw = twiddles(c, G.nx);
                 launch_row(G.nx, ROW_INV_T_FWD, pa, nact, G.ny, G.s);
                 pa.tw = twiddles(c, G.ny);

@@ -244,4 +244,78 @@ __device__ __forceinline__ void team_fft(float2 (&v)[N / G], int g, const float2
     }
 }
 
+// ---------------------------------------------------------------------------
+// 2048 points on a team of 64 threads, 32 points each.  The two-level scheme above needs 64 points per
+// thread, which leaves room for 8 warps per SM; this one runs 16 and pays half a transpose and one
+// twiddle layer more.  3 waves of 2048^2: row step 78.0 -> 64.7 us, column step 108 -> 98, both in turn
+// 210 -> 162; one wave 73.9 -> 55.1; the same error against 64 bits (2.1e-7 per slice, 3.87e-6 after
+// 240).  2048 = 32 x 8 x 8:
+//   1. thread g holds x[g + 64 j] (j < 32): 32-point DFT over j, twiddle W_2048^(g k1);
+//   2. transpose (k1, g) so that thread t holds k1 = t mod 32 and, of g = 8 a + b, every a for the
+//      four b = t / 32 + 2 m: 8-point DFTs over a, twiddle W_64^(b c);
+//   3. threads t and t xor 32 share k1: each gives the other the half of its values whose c has the
+//      other's parity, then holds every b for c = t / 32 + 2 m: 8-point DFTs over b give
+//      X[k1 + 32 c + 256 d] = X[t + 64 (m + 4 d)], the input's distribution.
+// `scr(k1, g)` is the transpose's slot, `xch(q, t)` a slot of the exchange (q < 16, may overlap scr);
+// `sync()` orders the 64 threads.
+// ---------------------------------------------------------------------------
+// the twiddles W_64^(b c) of the four b = P + 2 m, carried as hi + lo
+template <int P, int DIR>
+__device__ __forceinline__ void team64_twiddle(float2 (&u)[4][8])
+{
+#pragma unroll
+    for (int m = 0; m < 4; m++)
+#pragma unroll
+        for (int c = 1; c < 8; c++) u[m][brev<8>(c)] = tw_apply<DIR>(u[m][brev<8>(c)], ((P + 2 * m) * c) & 63);
+}
+template <int DIR, class Scr, class Xch, class Sync>
+__device__ __forceinline__ void team64_fft(float2 (&v)[32], int t, const float2* __restrict__ tw, Scr scr, Xch xch,
+                                           Sync sync)
+{
+    constexpr int D = DIR < 0 ? -1 : 1;
+    dft_reg<32, D>(v);
+#pragma unroll
+    for (int k1 = 1; k1 < 32; k1++) {
+        const float2 w = tw[k1 * 64 + t];
+        float2& x = v[brev<32>(k1)];
+        x = DIR < 0 ? cmul(x, w) : cmulc_mirror(x, w);
+    }
+    sync();
+#pragma unroll
+    for (int k1 = 0; k1 < 32; k1++) *scr(k1, t) = v[brev<32>(k1)];
+    sync();
+    const int k1 = t & 31, p = t >> 5;
+    float2 u[4][8];
+#pragma unroll
+    for (int m = 0; m < 4; m++)
+#pragma unroll
+        for (int a = 0; a < 8; a++) u[m][a] = *scr(k1, 8 * a + 2 * m + p);
+#pragma unroll
+    for (int m = 0; m < 4; m++) dft_reg<8, D>(u[m]);
+    if (p == 0) team64_twiddle<0, D>(u);
+    else team64_twiddle<1, D>(u);
+    sync();
+    // u[m][brev(c)] is value (b = p + 2 m, c); give those with c of the other parity
+#pragma unroll
+    for (int m = 0; m < 4; m++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) *xch(4 * m + i, t) = p == 0 ? u[m][brev<8>(2 * i + 1)] : u[m][brev<8>(2 * i)];
+    sync();
+    // w[b] for c = p + 2 i: the own b = p + 2 m and the partner's b = 1 - p + 2 m
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        float2 w[8];
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            const float2 own = p == 0 ? u[m][brev<8>(2 * i)] : u[m][brev<8>(2 * i + 1)];
+            const float2 oth = *xch(4 * m + i, t ^ 32);
+            w[2 * m] = p == 0 ? own : oth;
+            w[2 * m + 1] = p == 0 ? oth : own;
+        }
+        dft_reg<8, D>(w);
+#pragma unroll
+        for (int d = 0; d < 8; d++) v[i + 4 * d] = w[brev<8>(d)];
+    }
+}
+
 }  // namespace msb

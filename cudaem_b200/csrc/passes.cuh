@@ -1006,6 +1006,135 @@ static bool col_pipe(const PassArgs& a, int nwaves, int nx, cudaStream_t st)
     }
 }
 
+// The 2048-point slice steps (instantiated by the 2048-point unit only)
+//
+// Row step of 2048 points, one row per 64-thread block (team64_fft): k_row_tt's operations, on either
+// store (SV: a σV store)
+template <int MODE, bool SV>
+__global__ void __launch_bounds__(64, 8) k_row_2048(PassArgs a)
+{
+    constexpr int N = 2048;
+    __shared__ float2 smem[32 * 65];
+    const int ny = a.grid.ny;
+    const int b = blockIdx.x / ny, r = blockIdx.x % ny, t = threadIdx.x;
+    chain_wait();
+    const bool beyond = a.slice >= a.waves[b].n_slices;
+    if (beyond && !(a.flags & PF_VACUUM_BEYOND)) return;
+    float2 v[32];
+    {
+        const float2* src = a.psi + ((size_t)b * ny + r) * N + t;
+#pragma unroll
+        for (int j = 0; j < 32; j++) v[j] = src[64 * j];
+    }
+    const float2* tw = a.tw64 + (size_t)((unsigned)a.slice % (unsigned)kTwSets) * N;   // through L1
+    auto scr = [&](int k1, int g) { return smem + k1 * 65 + g; };
+    auto xch = [&](int q, int g) { return smem + q * 64 + g; };
+    auto sync = []() { __syncthreads(); };
+    team64_fft<2>(v, t, tw, scr, xch, sync);
+    if (!beyond) {
+        const WaveInfo* wi = opaque(a.waves + b);
+        const size_t voff = ((size_t)(a.slice - a.sV_slice_base) * ny + r) * N + t;
+        if constexpr (SV) {
+            const float* vr = (wi->sV ? wi->sV : opaque(a.sV) + (size_t)wi->conf_slot * a.sV_slot_stride) + voff;
+#pragma unroll
+            for (int j = 0; j < 32; j++) v[j] = cmul(v[j], expi_tab(__ldg(vr + 64 * j), a.exptab));
+        } else {
+            const float2* tr = opaque(a.tt) + (size_t)wi->conf_slot * a.sV_slot_stride + voff;
+            const uint64_t pol = l2_policy_trans(MODE);
+#pragma unroll
+            for (int j = 0; j < 32; j++) v[j] = cmul(v[j], ld_nc_l2hint(tr + 64 * j, pol));
+        }
+    }
+    team64_fft<-1>(v, t, tw, scr, xch, sync);
+    chain_trigger();
+    float2* dst = opaque(a.psi) + ((size_t)b * ny + r) * N + t;
+    const uint64_t pol = l2_policy_wave(MODE);
+#pragma unroll
+    for (int j = 0; j < 32; j++) st_l2hint(dst + 64 * j, v[j], pol);
+}
+
+// Column step of 2048 points: four columns per block, 64 threads each (team64_fft), the tile brought in
+// by TMA as in k_col_step_tma.  Two blocks of four columns per SM time as one of eight (162 and 166 us
+// per slice for 3 waves, 389 and 387 for 8).
+constexpr int kCol2048 = 4;
+template <int TC>
+__global__ void __launch_bounds__(64 * TC, 2) k_col_2048(PassArgs a, const __grid_constant__ CUtensorMap tmap)
+{
+    constexpr int N = 2048, BOX = 256;
+    constexpr unsigned TILE_BYTES = (unsigned)(N * TC * sizeof(float2));
+    // columns start 16 / TC slots apart modulo 16, so a half-warp (TC columns x 16 / TC threads) is conflict-free
+    constexpr int SC = 32 * 65 + 16 / TC;
+    __shared__ __align__(8) uint64_t bar;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float2* smem = reinterpret_cast<float2*>(smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u));
+    const int nx = a.grid.nx;
+    const int tiles = nx / TC;
+    const int b = blockIdx.x / tiles;
+    const int col0 = (blockIdx.x % tiles) * TC;
+    const int c = threadIdx.x % TC, t = threadIdx.x / TC;
+    const int col = col0 + c;
+    const WaveInfo& wi = a.waves[b];
+    if (a.slice >= wi.n_slices && !(a.flags & PF_VACUUM_BEYOND)) {
+        chain_wait();
+        return;
+    }
+    const bool final_step = (a.slice == wi.n_slices - 1) && !(a.flags & PF_PROP_ALWAYS);
+    if (threadIdx.x == 0) mbar_init(&bar, 1);
+    chain_wait();
+    if (threadIdx.x == 0) {
+        mbar_expect_tx(&bar, TILE_BYTES + ((a.flags & PF_TEST_WAIT) ? 16u : 0u));
+#pragma unroll
+        for (int q = 0; q < N / BOX; q++) tma_load_2d(smem + q * BOX * TC, &tmap, 2 * col0, b * N + q * BOX, &bar);
+    }
+    __syncthreads();
+    const long long limit = (a.flags & PF_TEST_WAIT) ? 2000000LL : (a.wait_cycles > 0 ? a.wait_cycles : kWaitCycles);
+    const bool late = !mbar_wait_bounded(&bar, 0, limit);
+    if (__syncthreads_or(late)) {
+        if (threadIdx.x == 0 && a.err) atomicOr(a.err, 1);
+        return;
+    }
+    float2 v[32];
+#pragma unroll
+    for (int j = 0; j < 32; j++) v[j] = smem[(t + 64 * j) * TC + c];
+    float2* sb = smem + c * SC;
+    const float2* tw = a.tw64 + (size_t)((unsigned)a.slice % (unsigned)kTwSets) * N;
+    auto scr = [sb](int k1, int g) { return sb + k1 * 65 + g; };
+    auto xch = [sb](int q, int g) { return sb + q * 64 + g; };
+    auto sync = []() { __syncthreads(); };
+    team64_fft<-1>(v, t, tw, scr, xch, sync);
+    const size_t cs = (size_t)64 * nx;
+    if (!final_step) {
+        const float2* pp = opaque(prop_set(wi.prop ? wi.prop : a.prop, a) + (size_t)t * nx + col);
+        const uint64_t pl = l2_policy_evict_last();
+#pragma unroll
+        for (int j = 0; j < 32; j++) v[j] = cmul(v[j], ld_nc_l2hint(pp + j * cs, pl));
+        team64_fft<2>(v, t, tw, scr, xch, sync);
+    }
+    chain_trigger();
+    float2* cp = opaque(a.psi + (size_t)b * N * nx + (size_t)t * nx + col);
+    const uint64_t pol = l2_policy_wave(a.l2_mode);
+#pragma unroll
+    for (int j = 0; j < 32; j++) st_l2hint(cp + j * cs, v[j], pol);
+}
+[[maybe_unused]] static bool col_2048(const PassArgs& a, int nwaves, int nx, cudaStream_t st)
+{
+    constexpr int TC = kCol2048;
+    if (((uintptr_t)a.psi & 15) != 0) return false;
+    CUtensorMap map;
+    if (!encode_wave_tile_map(&map, a.psi, nx, (int64_t)nwaves * 2048, 2 * TC, 256)) return false;
+    const size_t sm = sizeof(float2) * TC * (32 * 65 + 16 / TC) + 128;
+    smem_attr(k_col_2048<TC>, sm);
+    launch_step(k_col_2048<TC>, (unsigned)(nwaves * (nx / TC)), 64 * TC, sm, st, a.chained != 0, a, map);
+    return true;
+}
+
+template <int MODE>
+static void row_2048(const PassArgs& a, int nwaves, int ny, cudaStream_t st)
+{
+    if (a.tt) launch_step(k_row_2048<MODE, false>, (unsigned)(nwaves * ny), 64, 0, st, a.chained != 0, a);
+    else launch_step(k_row_2048<MODE, true>, (unsigned)(nwaves * ny), 64, 0, st, a.chained != 0, a);
+}
+
 template <int N>
 void row_dispatch(int op, const PassArgs& a, int nwaves, int ny, cudaStream_t st)
 {
@@ -1044,6 +1173,15 @@ void row_dispatch(int op, const PassArgs& a, int nwaves, int ny, cudaStream_t st
         else if (a.tt) wide_step(k_row_tt<N, L2_DEFAULT, L, false, ROWF_ADJOINT>);
         else wide_step(k_row_tt<N, L2_DEFAULT, L, true, ROWF_ADJOINT>);
         return;
+    }
+    if constexpr (N == 2048) {
+        // the 64-thread teams, where the call allows them (PassArgs.tw64), on every tile shape
+        if (op == ROW_INV_T_FWD && a.tw64) {
+            if (a.l2_mode == L2_WAVES_RESIDENT) row_2048<L2_WAVES_RESIDENT>(a, nwaves, ny, st);
+            else if (a.l2_mode == L2_SHARED_T) row_2048<L2_SHARED_T>(a, nwaves, ny, st);
+            else row_2048<L2_DEFAULT>(a, nwaves, ny, st);
+            return;
+        }
     }
     if (op == ROW_INV_T_FWD && a.tt) {
         if (narrow)
@@ -1093,6 +1231,8 @@ void col_dispatch(int op, const PassArgs& a, int nwaves, int nx, cudaStream_t st
         return;
     // the hot column step reads its tile through the tensor memory accelerator
     if (op == COL_STEP && a.variant != PASS_PIPELINED && !(a.flags & PF_FILTER_AUX)) {
+        if constexpr (N == 2048)
+            if (a.tw64 && !(a.flags & PF_CONJ_PROP) && col_2048(a, nwaves, nx, st)) return;
         if ((a.tile & TILE_WARP_COLS) && col_step_warp<N>(a, nwaves, nx, st)) return;
         if ((a.tile & TILE_NARROW_COLS) && col_step_tma<N, NarrowLayout<N>>(a, nwaves, nx, st)) return;
         if (col_step_tma<N>(a, nwaves, nx, st)) return;
