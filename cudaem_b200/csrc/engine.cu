@@ -222,6 +222,33 @@ const float2* twiddles64(ms_ctx* c, int nx, int ny)
     return nx == 2048 || ny == 2048 ? twiddles(c, 2048, 64) : nullptr;
 }
 
+// Twiddles of the short steps, hi + lo: W_N^(t k1) at [k1][t], then W_T^(b c) at [b][c]; null for
+// lengths that have none.
+const float4* short_twiddles(ms_ctx* c, int N)
+{
+    if (N > 512) return nullptr;
+    const int key = N + 1;   // beside the even keys of the other tables
+    auto it = c->twiddles.find(key);
+    if (it != c->twiddles.end()) return (const float4*)it->second;
+    const int T = N / 8, RA = N == 128 ? 4 : 8, RB = T / RA;
+    std::vector<float4> t((size_t)N + T);
+    auto put = [&](size_t i, double num, double den) {
+        const double a = -2.0 * kPi * num / den, x = std::cos(a), y = std::sin(a);
+        const float hx = (float)x, hy = (float)y;
+        t[i] = make_float4(hx, hy, (float)(x - hx), (float)(y - hy));
+    };
+    for (int k1 = 0; k1 < 8; k1++)
+        for (int g = 0; g < T; g++) put((size_t)k1 * T + g, (double)(g * k1), (double)N);
+    for (int b = 0; b < RB; b++)
+        for (int k = 0; k < RA; k++) put((size_t)N + b * RA + k, (double)(b * k), (double)T);
+    void* p = nullptr;
+    CK(cudaMalloc(&p, sizeof(float4) * t.size()));
+    c->forget_free_mem();
+    CK(cudaMemcpy(p, t.data(), sizeof(float4) * t.size(), cudaMemcpyHostToDevice));
+    c->twiddles[key] = p;
+    return (const float4*)p;
+}
+
 LensDev lens_dev(const LensCoef& L)
 {
     LensDev d;
@@ -301,6 +328,7 @@ struct Setup {
     GridDev gd;
     const float2* tw_x;
     const float2* tw_y;
+    const float4 *short_x, *short_y;
     const float2* tw64;
     const float2* prop;
     const float2* propT = nullptr;   // transposed propagator tables (1024-point columns), or null
@@ -334,6 +362,8 @@ Setup make_setup(ms_ctx* c, const ms_params& p)
     s.gd.g0y = s.gc.g0y;
     s.tw_x = twiddles(c, p.nx);
     s.tw_y = twiddles(c, p.ny);
+    s.short_x = short_twiddles(c, p.nx);
+    s.short_y = short_twiddles(c, p.ny);
     s.tw64 = twiddles64(c, p.nx, p.ny);
     // full table P(k), rebuilt only when the grid, wavelength, slice thickness or tilt change
     char key[256];
@@ -1138,6 +1168,13 @@ void sim_tem_like(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* o
         PassArgs pa = pass_args(s, psi, dwv, sVs, slot, cond);
         pa.l2_mode = l2_mode_for_waves(nw, N);
         pa.tt = sT;
+        if (!force_cbed && p.simulation_type != MS_SIM_CBED) {
+            // small batches take the short steps.  (CBED keeps the transforms it shares with an uneven
+            // batch, so that a simulation gives the same values alone and in one; STEM keeps the
+            // same for full and partial probe batches.)
+            pa.short_x = s.short_x;
+            pa.short_y = s.short_y;
+        }
         pa.tile = choose_tile(c, pa, p.nx, p.ny, nw, g.S_cap, st);
         c->last_tile = pa.tile;
         if (iw == MS_IW_CONVERGENT) {
@@ -1752,6 +1789,8 @@ void sim_thickness(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* 
         pa.aux_stride = (int64_t)chunk * N;
         pa.filt_g2in = g2in;
         pa.filt_g2out = g2out;
+        pa.short_x = s.short_x;
+        pa.short_y = s.short_y;
         pa.tile = choose_tile(c, pa, p.nx, p.ny, nw, g.S_cap, st);
         c->last_tile = pa.tile;
         const bool chain = chain_steps(c, nw, N);
@@ -2003,7 +2042,8 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
         upload(c, dwv, wv.data(), sizeof(WaveInfo) * nb, st);
         PassArgs pa = pass_args(s, adj, dwv, sV, slot, cond);
         pa.tt = sT;
-        pa.tw64 = nullptr;   // the adjoint's row and column steps are those of the 32-thread teams
+        // forward, recomputed and adjoint steps are those whose transforms the adjoint kernels share
+        pa.tw64 = nullptr;
         pa.l2_mode = l2_mode_for_waves(nb, N);
         pa.tile = choose_tile(c, pa, p.nx, p.ny, nb, S, st);
         pa.det_thr = dthr;

@@ -318,4 +318,70 @@ __device__ __forceinline__ void team64_fft(float2 (&v)[32], int t, const float2*
     }
 }
 
+// ---------------------------------------------------------------------------
+// Short steps for small batches: N = 512, 256 or 128 points on T = N / 8 threads, 8 points each.  A
+// batch of one or two waves leaves most of the GPU idle with 16 or 32 points per thread, and a step
+// takes as long as one thread's chain of operations; this form has a quarter of the chain and four
+// times the threads, for one transpose more.  N = 8 x RA x RB with T = RA RB:
+//   1. thread t holds x[t + T j]: 8-point DFT over j, twiddle W_N^(t k1);
+//   2. transpose; k1 = t mod 8 and, of t' = RB a + b, every a: RA-point DFTs, twiddle W_T^(b c);
+//   3. transpose; every b of a c: RB-point DFTs give X[k1 + 8 c + 8 RA d], the input's distribution.
+// Both twiddles are carried as hi + lo (`tw`: N entries at [k1][t], then T at [b][c]).
+// Per slice of one wave, chained: 512^2 10.6 -> 6.4 us, 256^2 5.9 -> 5.2, 128^2 6.3 -> 4.7; two waves
+// 512^2 12.3 -> 9.2; but four 15.2 -> 16.4, and eight of 256^2 8.6 -> 9.3.
+// ---------------------------------------------------------------------------
+template <int DIR>
+__device__ __forceinline__ float2 short_twiddle(float2 x, float4 w)
+{
+    const float2 hi = make_float2(w.x, w.y), lo = make_float2(w.z, w.w);
+    return DIR < 0 ? cmul_split(x, hi, lo) : cmulc_split(x, hi, lo);
+}
+template <int N, int DIR, class Scr, class Sync>
+__device__ __forceinline__ void short_fft(float2 (&v)[8], int t, const float4* __restrict__ tw, Scr scr, Sync sync)
+{
+    using S = ShortCfg<N>;
+    constexpr int T = S::T, RA = S::RA, RB = S::RB, MA = 8 / RA, MB = 8 / RB;
+    dft_reg<8, DIR>(v);
+#pragma unroll
+    for (int k1 = 1; k1 < 8; k1++) {
+        v[brev<8>(k1)] = short_twiddle<DIR>(v[brev<8>(k1)], __ldg(tw + k1 * T + t));
+    }
+    sync();
+#pragma unroll
+    for (int k1 = 0; k1 < 8; k1++) *scr(k1, t) = v[brev<8>(k1)];
+    sync();
+    // this thread: k1 = t mod 8, and of t' = RB a + b every a for b = t / 8 + (T / 8) m
+    const int k1 = t & 7, q = t >> 3;
+    float2 u[MA][RA];
+#pragma unroll
+    for (int m = 0; m < MA; m++)
+#pragma unroll
+        for (int a = 0; a < RA; a++) u[m][a] = *scr(k1, RB * a + q + (T / 8) * m);
+#pragma unroll
+    for (int m = 0; m < MA; m++) {
+        dft_reg<RA, DIR>(u[m]);
+#pragma unroll
+        for (int c = 1; c < RA; c++) {
+            float2& x = u[m][brev<RA>(c)];
+            x = short_twiddle<DIR>(x, __ldg(tw + N + (q + (T / 8) * m) * RA + c));
+        }
+    }
+    sync();
+#pragma unroll
+    for (int m = 0; m < MA; m++)
+#pragma unroll
+        for (int c = 0; c < RA; c++) *scr(k1, RB * c + q + (T / 8) * m) = u[m][brev<RA>(c)];
+    sync();
+    // every b for c = t / 8 + (T / 8) m: X[k1 + 8 c + 8 RA d] = X[t + T (m + MB d)]
+#pragma unroll
+    for (int m = 0; m < MB; m++) {
+        float2 w[RB];
+#pragma unroll
+        for (int b = 0; b < RB; b++) w[b] = *scr(k1, RB * (q + (T / 8) * m) + b);
+        dft_reg<RB, DIR>(w);
+#pragma unroll
+        for (int d = 0; d < RB; d++) v[m + MB * d] = w[brev<RB>(d)];
+    }
+}
+
 }  // namespace msb

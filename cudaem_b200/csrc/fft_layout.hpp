@@ -72,6 +72,25 @@ struct NarrowCfg {
     static constexpr int TC = N < 256 ? 32 / G : 4;
 };
 
+// Short steps (fft.cuh): T = N / 8 threads per transform, N = 8 RA RB
+template <int N>
+struct ShortCfg;
+template <>
+struct ShortCfg<512> {
+    static constexpr int T = 64, RA = 8, RB = 8;
+};
+template <>
+struct ShortCfg<256> {
+    static constexpr int T = 32, RA = 8, RB = 4;
+};
+template <>
+struct ShortCfg<128> {
+    static constexpr int T = 16, RA = 4, RB = 4;
+};
+// The batches they serve, in wave pixels: up to two waves of 512^2; shorter transforms have fewer
+// points per thread to begin with, and lose from 2^18 pixels on (figures in fft.cuh)
+inline bool short_step(int N, long long pixels) { return N <= 512 && pixels <= (N == 512 ? 1 << 19 : 1 << 17); }
+
 template <int N, int ROWS_ = FftCfg<N>::ROWS, int TC_ = FftCfg<N>::TC>
 struct FftLayoutT {
     static constexpr int G = FftCfg<N>::G;

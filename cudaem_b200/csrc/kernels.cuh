@@ -87,6 +87,8 @@ struct PassArgs {
     int64_t sV_slot_stride;   // elements per slot
     int sV_slice_base;        // slice index held at the store's slice 0
     const float2* tw;         // inter-level twiddles for this pass's length
+    const float4* short_x;    // twiddles of the short steps for rows and columns (fft.cuh), or null: not used
+    const float4* short_y;
     const float2* tw64;       // those of 2048 points on teams of 64 threads, or null: the slice steps of
                               // that length run on teams of 32 (gradient calls, whose bits stay)
     const float2* prop_x;     // [nx] exp(i w (gx - g0x)^2)

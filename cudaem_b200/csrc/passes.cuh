@@ -1135,6 +1135,128 @@ static void row_2048(const PassArgs& a, int nwaves, int ny, cudaStream_t st)
     else launch_step(k_row_2048<MODE, true>, (unsigned)(nwaves * ny), 64, 0, st, a.chained != 0, a);
 }
 
+// The slice steps of small batches (short_fft), bound by latency: the slice's transmission and the
+// propagator, which no step writes, are read before the wait for the step ahead.  Rows: blocks of 64
+// threads, one row of 512 points or several shorter ones.  Columns: four per block (32-byte row
+// segments), by ordinary loads.  FILT: the propagated spectrum inside the annulus also goes to
+// PassArgs.aux.
+constexpr int kShortThreads = 64, kShortCols = 4;
+template <int N, bool SV>
+__global__ void __launch_bounds__(kShortThreads) k_row_short(PassArgs a)
+{
+    constexpr int T = ShortCfg<N>::T, R = kShortThreads / T;
+    constexpr int P = T + 1, SR = 8 * P + 1;
+    __shared__ float2 smem[R * SR];
+    const int ny = a.grid.ny;
+    const int team = threadIdx.x / T, t = threadIdx.x % T;
+    const int row = blockIdx.x * R + team, b = row / ny, r = row % ny;
+    const bool beyond = a.slice >= a.waves[b].n_slices;
+    const WaveInfo& wi = a.waves[b];
+    float2 x[8];
+    if (!beyond) {
+        const size_t voff = ((size_t)(a.slice - a.sV_slice_base) * ny + r) * N + t;
+        if constexpr (SV) {
+            const float* vr = (wi.sV ? wi.sV : a.sV + (size_t)wi.conf_slot * a.sV_slot_stride) + voff;
+#pragma unroll
+            for (int j = 0; j < 8; j++) x[j] = expi_tab(__ldg(vr + T * j), a.exptab);
+        } else {
+            const float2* tr = a.tt + (size_t)wi.conf_slot * a.sV_slot_stride + voff;
+#pragma unroll
+            for (int j = 0; j < 8; j++) x[j] = __ldg(tr + T * j);
+        }
+    }
+    chain_wait();
+    if (beyond && !(a.flags & PF_VACUUM_BEYOND)) return;
+    float2* p = a.psi + (size_t)row * N + t;
+    float2 v[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = p[T * j];
+    float2* sb = smem + team * SR;
+    auto scr = [sb](int k1, int g) { return sb + k1 * P + g; };
+    auto sync = []() { if (T > 32) __syncthreads(); else __syncwarp(); };
+    short_fft<N, +1>(v, t, a.short_x, scr, sync);
+    if (!beyond) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) v[j] = cmul(v[j], x[j]);
+    }
+    short_fft<N, -1>(v, t, a.short_x, scr, sync);
+    chain_trigger();
+#pragma unroll
+    for (int j = 0; j < 8; j++) p[T * j] = v[j];
+}
+template <int N, bool FILT>
+__global__ void __launch_bounds__(kShortCols * ShortCfg<N>::T) k_col_short(PassArgs a)
+{
+    constexpr int T = ShortCfg<N>::T, TC = kShortCols;
+    constexpr int P = T + 1, SC = (8 * P + 15) / 16 * 16 + 4;
+    __shared__ float2 smem[TC * SC];
+    const int nx = a.grid.nx, tiles = nx / TC;
+    const int b = blockIdx.x / tiles, col = (blockIdx.x % tiles) * TC + threadIdx.x % TC, t = threadIdx.x / TC;
+    const WaveInfo& wi = a.waves[b];
+    const bool skip = a.slice >= wi.n_slices && !(a.flags & PF_VACUUM_BEYOND);
+    const bool final_step = (a.slice == wi.n_slices - 1) && !(a.flags & PF_PROP_ALWAYS);
+    const size_t cs = (size_t)T * nx;
+    float2 x[8];
+    const float2* pp = prop_set(wi.prop ? wi.prop : a.prop, a) + (size_t)t * nx + col;
+#pragma unroll
+    for (int j = 0; j < 8; j++) x[j] = __ldg(pp + j * cs);
+    chain_wait();
+    if (skip) return;
+    float2* p = a.psi + (size_t)b * N * nx + (size_t)t * nx + col;
+    float2 v[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = p[j * cs];
+    float2* sb = smem + (threadIdx.x % TC) * SC;
+    auto scr = [sb](int k1, int g) { return sb + k1 * P + g; };
+    auto sync = []() { __syncthreads(); };
+    short_fft<N, -1>(v, t, a.short_y, scr, sync);
+    if (!final_step) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) v[j] = cmul(v[j], x[j]);
+        if constexpr (FILT) {
+            float2* ab = a.aux + (size_t)b * a.aux_stride + (size_t)t * nx + col;
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const float g2 = det_g2(col, t + T * j, nx, N, a.grid.dgx_f, a.grid.dgy_f);
+                ab[j * cs] = (a.filt_g2in <= g2 && g2 <= a.filt_g2out) ? v[j] : make_float2(0.0f, 0.0f);
+            }
+        }
+        short_fft<N, +1>(v, t, a.short_y, scr, sync);
+    }
+    chain_trigger();
+#pragma unroll
+    for (int j = 0; j < 8; j++) p[j * cs] = v[j];
+}
+
+template <int N>
+static bool row_short(const PassArgs& a, int nwaves, int ny, cudaStream_t st)
+{
+    if constexpr (N > 512) {
+        return false;
+    } else {
+        if (!a.short_x || a.variant == PASS_PIPELINED || !short_step(N, (long long)nwaves * ny * N)) return false;
+        auto kern = a.tt ? k_row_short<N, false> : k_row_short<N, true>;
+        launch_step(kern, (unsigned)((size_t)nwaves * ny * ShortCfg<N>::T / kShortThreads), kShortThreads, 0, st,
+                    a.chained != 0, a);
+        return true;
+    }
+}
+template <int N>
+static bool col_short(const PassArgs& a, int nwaves, int nx, cudaStream_t st)
+{
+    if constexpr (N > 512) {
+        return false;
+    } else {
+        // (an injected wait fault needs the step that waits for a tile)
+        if (!a.short_y || a.variant == PASS_PIPELINED || (a.flags & (PF_CONJ_PROP | PF_TEST_WAIT)) ||
+            !short_step(N, (long long)nwaves * nx * N))
+            return false;
+        auto kern = (a.flags & PF_FILTER_AUX) ? k_col_short<N, true> : k_col_short<N, false>;
+        launch_step(kern, (unsigned)(nwaves * (nx / kShortCols)), kShortCols * ShortCfg<N>::T, 0, st, a.chained != 0, a);
+        return true;
+    }
+}
+
 template <int N>
 void row_dispatch(int op, const PassArgs& a, int nwaves, int ny, cudaStream_t st)
 {
@@ -1174,6 +1296,8 @@ void row_dispatch(int op, const PassArgs& a, int nwaves, int ny, cudaStream_t st
         else wide_step(k_row_tt<N, L2_DEFAULT, L, true, ROWF_ADJOINT>);
         return;
     }
+    // small batches, on every tile shape
+    if (op == ROW_INV_T_FWD && row_short<N>(a, nwaves, ny, st)) return;
     if constexpr (N == 2048) {
         // the 64-thread teams, where the call allows them (PassArgs.tw64), on every tile shape
         if (op == ROW_INV_T_FWD && a.tw64) {
@@ -1229,6 +1353,7 @@ void col_dispatch(int op, const PassArgs& a, int nwaves, int nx, cudaStream_t st
     if (op == COL_STEP && a.variant == PASS_PIPELINED && !(a.flags & PF_FILTER_AUX) && ((uintptr_t)a.prop & 15) == 0 &&
         col_pipe<N>(a, nwaves, nx, st))
         return;
+    if (op == COL_STEP && col_short<N>(a, nwaves, nx, st)) return;
     // the hot column step reads its tile through the tensor memory accelerator
     if (op == COL_STEP && a.variant != PASS_PIPELINED && !(a.flags & PF_FILTER_AUX)) {
         if constexpr (N == 2048)
