@@ -1939,18 +1939,27 @@ void sim_stem_forward_potential(ms_ctx* c, const ms_params& p, const float* V, i
         // the tile shape is tuned as for the simulations, and the waves stay in L2 where they fit
         pa.l2_mode = l2_mode_for_waves(nb, N);
         pa.tile = choose_tile(c, pa, p.nx, p.ny, nb, S, st);
-        pa.tw = s.tw_y;
-        run_col(c, p.ny, COL_PROBE_INV, pa, nb, p.nx, st);
-        pa.chained = chain_steps(c, nb, N);
-        for (int sl = 0; sl < S; sl++) {
-            pa.slice = sl;
-            pa.tw = s.tw_x;
-            run_row(c, p.nx, ROW_INV_T_FWD, pa, nb, p.ny, st);
-            pa.tw = s.tw_y;
-            run_col(c, p.ny, COL_STEP, pa, nb, p.nx, st);
-        }
-        launch_detect(psi, nb, p.nx, p.ny, s.gd.dgx_f, s.gd.dgy_f, dthr, dthr + ndet, ndet, partial, nblk, st);
-        launch_det_finalize(partial, nb, nblk, ndet, dwv, Iw + (int64_t)start * ndet, nullptr, 0, 0, st);
+        // on the transmission store the launches hold none of the caller's pointers, so the loop replays
+        // from a graph whatever buffers the next call brings
+        if (sT) pa.sV = nullptr;
+        double* Ib = Iw + (int64_t)start * ndet;
+        auto body = [&] {
+            PassArgs q = pa;
+            q.tw = s.tw_y;
+            run_col(c, p.ny, COL_PROBE_INV, q, nb, p.nx, st);
+            q.chained = chain_steps(c, nb, N);
+            for (int sl = 0; sl < S; sl++) {
+                q.slice = sl;
+                q.tw = s.tw_x;
+                run_row(c, p.nx, ROW_INV_T_FWD, q, nb, p.ny, st);
+                q.tw = s.tw_y;
+                run_col(c, p.ny, COL_STEP, q, nb, p.nx, st);
+            }
+            launch_detect(psi, nb, p.nx, p.ny, s.gd.dgx_f, s.gd.dgy_f, dthr, dthr + ndet, ndet, partial, nblk, st);
+            launch_det_finalize(partial, nb, nblk, ndet, dwv, Ib, nullptr, 0, 0, st);
+        };
+        if (sT) run_graphed(c, graph_key_of(pa, nb, S, nblk, ndet, partial, Ib, nullptr, dthr, -3), body);
+        else body();
         CK(cudaStreamSynchronize(st));
     }
     float* o = (float*)c->buf("stem_out", sizeof(float) * np * ndet);
@@ -2014,7 +2023,11 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
     // transmitted waves of two segments: the one being swept back and the one being recomputed
     float2* xseg = (float2*)c->buf("adj_xseg", sizeof(float2) * N * B * k * 2);
     float2* ckpt = nseg > 1 ? (float2*)c->buf("adj_ckpt", sizeof(float2) * N * B * (nseg - 1)) : nullptr;
-    float* gV = on_dev ? dV : (float*)c->buf("adj_dV", sizeof(float) * slot);
+    // The batch's launches replay from a graph when they hold none of the caller's pointers: on the
+    // transmission store, with the gradient summed in the context's memory and copied out at the end
+    // (where that takes at most a twentieth of the free memory).
+    const bool graphed = sT && (!on_dev || (double)slot * sizeof(float) <= 0.05 * (double)c->free_mem());
+    float* gV = on_dev && !graphed ? dV : (float*)c->buf("adj_dV", sizeof(float) * slot);
     float* gVw = (float*)c->buf("adj_dVw", sizeof(float) * N * B);   // per-wave planes of one slice
     double* partial = (double*)c->buf("det_part", sizeof(double) * B * nblk * ndet);
     double* Iw = (double*)c->buf("det_I", sizeof(double) * B * ndet);
@@ -2050,96 +2063,114 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
         pa.ndet = ndet;
         pa.resid = resid;
         pa.chi_part = chi_part;
-        // forward sweep with checkpoints
-        pa.tw = s.tw_y;
-        run_col(c, p.ny, COL_PROBE_INV, pa, nb, p.nx, st);
-        const int last0 = (nseg - 1) * k;
-        auto xbuf = [&](int seg) { return xseg + (int64_t)(seg % 2) * k * wstride; };
-        for (int sl = 0; sl < S; sl++) {
-            if (sl < last0 && sl % k == 0)
-                CK(cudaMemcpyAsync(ckpt + (int64_t)(sl / k) * wstride, adj, sizeof(float2) * wstride,
-                                   cudaMemcpyDeviceToDevice, st));
-            pa.slice = sl;
-            pa.flags = sl >= last0 ? PF_STORE_X : 0;
-            pa.xs = xbuf(nseg - 1) + (int64_t)(sl - last0) * wstride;
-            pa.tw = s.tw_x;
-            run_row(c, p.nx, ROW_INV_T_FWD, pa, nb, p.ny, st);
-            pa.flags = 0;
+        if (graphed) pa.sV = nullptr;
+        const PassArgs pa0 = pa;
+        auto body = [&] {
+            PassArgs pa = pa0;
+            // forward sweep with checkpoints
             pa.tw = s.tw_y;
-            run_col(c, p.ny, COL_STEP, pa, nb, p.nx, st);
-        }
-        launch_detect(adj, nb, p.nx, p.ny, s.gd.dgx_f, s.gd.dgy_f, dthr, dthr + ndet, ndet, partial, nblk, st);
-        launch_det_finalize(partial, nb, nblk, ndet, dwv, Iw, nullptr, 0, 0, st);
-        launch_resid(Iw, dtgt + (int64_t)start * ndet, nb * ndet, resid, sq + (int64_t)start * ndet, st);
-        pa.tw = s.tw_y;
-        run_col(c, p.ny, COL_SEED, pa, nb, p.nx, st);
-        // Segments are recomputed on a second stream one segment ahead of the backward sweep,
-        // into the other half of the transmitted-wave buffer; events order each recompute after
-        // the sweep that last read its half, and each sweep after its recompute.  With
-        // per-launch profiling on, everything runs in order on the context stream.
-        const bool two = !c->profile && nseg > 1;
-        cudaStream_t rs = two ? pot_stream(c) : st;
-        auto recompute = [&](int seg) {
-            const int c0 = seg * k, c1 = std::min(S, c0 + k);
-            PassArgs pr = pa;
-            pr.psi = ckpt + (int64_t)seg * wstride;   // in place on the segment's checkpoint
-            for (int sl = c0; sl < c1; sl++) {
-                pr.slice = sl;
-                pr.flags = PF_STORE_X;
-                pr.xs = xbuf(seg) + (int64_t)(sl - c0) * wstride;
-                pr.tw = s.tw_x;
-                run_row(c, p.nx, ROW_INV_T_FWD, pr, nb, p.ny, rs);
-                if (sl < c1 - 1) {
-                    pr.flags = 0;
-                    pr.tw = s.tw_y;
-                    run_col(c, p.ny, COL_STEP, pr, nb, p.nx, rs);
+            run_col(c, p.ny, COL_PROBE_INV, pa, nb, p.nx, st);
+            const int last0 = (nseg - 1) * k;
+            auto xbuf = [&](int seg) { return xseg + (int64_t)(seg % 2) * k * wstride; };
+            for (int sl = 0; sl < S; sl++) {
+                if (sl < last0 && sl % k == 0)
+                    CK(cudaMemcpyAsync(ckpt + (int64_t)(sl / k) * wstride, adj, sizeof(float2) * wstride,
+                                       cudaMemcpyDeviceToDevice, st));
+                pa.slice = sl;
+                pa.flags = sl >= last0 ? PF_STORE_X : 0;
+                pa.xs = xbuf(nseg - 1) + (int64_t)(sl - last0) * wstride;
+                pa.tw = s.tw_x;
+                run_row(c, p.nx, ROW_INV_T_FWD, pa, nb, p.ny, st);
+                pa.flags = 0;
+                pa.tw = s.tw_y;
+                run_col(c, p.ny, COL_STEP, pa, nb, p.nx, st);
+            }
+            launch_detect(adj, nb, p.nx, p.ny, s.gd.dgx_f, s.gd.dgy_f, dthr, dthr + ndet, ndet, partial, nblk, st);
+            launch_det_finalize(partial, nb, nblk, ndet, dwv, Iw, nullptr, 0, 0, st);
+            launch_resid(Iw, dtgt + (int64_t)start * ndet, nb * ndet, resid, sq + (int64_t)start * ndet, st);
+            pa.tw = s.tw_y;
+            run_col(c, p.ny, COL_SEED, pa, nb, p.nx, st);
+            // Segments are recomputed on a second stream one segment ahead of the backward sweep,
+            // into the other half of the transmitted-wave buffer; events order each recompute after
+            // the sweep that last read its half, and each sweep after its recompute.  With
+            // per-launch profiling on, everything runs in order on the context stream.
+            const bool two = !c->profile && nseg > 1;
+            cudaStream_t rs = two ? pot_stream(c) : st;
+            auto recompute = [&](int seg) {
+                const int c0 = seg * k, c1 = std::min(S, c0 + k);
+                PassArgs pr = pa;
+                pr.psi = ckpt + (int64_t)seg * wstride;   // in place on the segment's checkpoint
+                for (int sl = c0; sl < c1; sl++) {
+                    pr.slice = sl;
+                    pr.flags = PF_STORE_X;
+                    pr.xs = xbuf(seg) + (int64_t)(sl - c0) * wstride;
+                    pr.tw = s.tw_x;
+                    run_row(c, p.nx, ROW_INV_T_FWD, pr, nb, p.ny, rs);
+                    if (sl < c1 - 1) {
+                        pr.flags = 0;
+                        pr.tw = s.tw_y;
+                        run_col(c, p.ny, COL_STEP, pr, nb, p.nx, rs);
+                    }
+                }
+            };
+            auto ev_rec = [&](int seg) { return chunk_event(c, (size_t)(2 * seg)); };
+            auto ev_back = [&](int seg) { return chunk_event(c, (size_t)(2 * seg + 1)); };
+            if (two) {
+                cudaEvent_t fwd_done = chunk_event(c, (size_t)(2 * nseg));
+                CK(cudaEventRecord(fwd_done, st));
+                CK(cudaStreamWaitEvent(rs, fwd_done, 0));
+                recompute(nseg - 2);
+                CK(cudaEventRecord(ev_rec(nseg - 2), rs));
+            }
+            for (int seg = nseg - 1; seg >= 0; seg--) {
+                const int c0 = seg * k, c1 = std::min(S, c0 + k);
+                if (seg != nseg - 1) {
+                    if (two) CK(cudaStreamWaitEvent(st, ev_rec(seg), 0));
+                    else recompute(seg);
+                }
+                for (int i = c1 - 1; i >= c0; i--) {
+                    pa.slice = i;
+                    pa.flags = 0;
+                    pa.xs = xbuf(seg) + (int64_t)(i - c0) * wstride;
+                    pa.dV = gVw;
+                    pa.tw = s.tw_x;
+                    run_row(c, p.nx, ROW_ADJ, pa, nb, p.ny, st);
+                    launch_sum_waves(gVw, nb, N, gV + (int64_t)i * N, st);
+                    pa.tw = s.tw_y;
+                    if (i > 0) {
+                        pa.slice = i - 1;
+                        pa.flags = PF_CONJ_PROP | PF_PROP_ALWAYS;
+                        run_col(c, p.ny, COL_STEP, pa, nb, p.nx, st);
+                    } else {
+                        run_col(c, p.ny, COL_GRAD_PROBE, pa, nb, p.nx, st);
+                        launch_chi_finalize(chi_part, nb, tiles, chi_acc, st);
+                    }
+                }
+                if (two && seg - 2 >= 0) {
+                    // the segment two below reuses this segment's half of the buffer
+                    CK(cudaEventRecord(ev_back(seg), st));
+                    CK(cudaStreamWaitEvent(rs, ev_back(seg), 0));
+                    recompute(seg - 2);
+                    CK(cudaEventRecord(ev_rec(seg - 2), rs));
                 }
             }
         };
-        auto ev_rec = [&](int seg) { return chunk_event(c, (size_t)(2 * seg)); };
-        auto ev_back = [&](int seg) { return chunk_event(c, (size_t)(2 * seg + 1)); };
-        if (two) {
-            cudaEvent_t fwd_done = chunk_event(c, (size_t)(2 * nseg));
-            CK(cudaEventRecord(fwd_done, st));
-            CK(cudaStreamWaitEvent(rs, fwd_done, 0));
-            recompute(nseg - 2);
-            CK(cudaEventRecord(ev_rec(nseg - 2), rs));
-        }
-        for (int seg = nseg - 1; seg >= 0; seg--) {
-            const int c0 = seg * k, c1 = std::min(S, c0 + k);
-            if (seg != nseg - 1) {
-                if (two) CK(cudaStreamWaitEvent(st, ev_rec(seg), 0));
-                else recompute(seg);
-            }
-            for (int i = c1 - 1; i >= c0; i--) {
-                pa.slice = i;
-                pa.flags = 0;
-                pa.xs = xbuf(seg) + (int64_t)(i - c0) * wstride;
-                pa.dV = gVw;
-                pa.tw = s.tw_x;
-                run_row(c, p.nx, ROW_ADJ, pa, nb, p.ny, st);
-                launch_sum_waves(gVw, nb, N, gV + (int64_t)i * N, st);
-                pa.tw = s.tw_y;
-                if (i > 0) {
-                    pa.slice = i - 1;
-                    pa.flags = PF_CONJ_PROP | PF_PROP_ALWAYS;
-                    run_col(c, p.ny, COL_STEP, pa, nb, p.nx, st);
-                } else {
-                    run_col(c, p.ny, COL_GRAD_PROBE, pa, nb, p.nx, st);
-                    launch_chi_finalize(chi_part, nb, tiles, chi_acc, st);
-                }
-            }
-            if (two && seg - 2 >= 0) {
-                // the segment two below reuses this segment's half of the buffer
-                CK(cudaEventRecord(ev_back(seg), st));
-                CK(cudaStreamWaitEvent(rs, ev_back(seg), 0));
-                recompute(seg - 2);
-                CK(cudaEventRecord(ev_rec(seg - 2), rs));
-            }
+        if (graphed) {
+            // the side stream and the events exist before a capture uses them
+            pot_stream(c);
+            chunk_event(c, (size_t)(2 * nseg));
+            std::string key = graph_key_of(pa0, nb, S, nblk, ndet, partial, Iw, dtgt + (int64_t)start * ndet, dthr, -4);
+            const void* ptrs[] = {xseg, ckpt, gV, gVw, resid, sq + (int64_t)start * ndet, chi_part, chi_acc};
+            key.append((const char*)ptrs, sizeof(ptrs));
+            key.append((const char*)&k, sizeof(k));
+            run_graphed(c, key, body);
+        } else {
+            body();
         }
         CK(cudaStreamSynchronize(st));  // the host wave table is refilled by the next batch
     }
-    if (!on_dev) CK(cudaMemcpyAsync(dV, gV, sizeof(float) * slot, cudaMemcpyDeviceToHost, st));
+    if (dV != gV)
+        CK(cudaMemcpyAsync(dV, gV, sizeof(float) * slot, on_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
     std::vector<double> hsq((size_t)np * ndet);
     double hchi[2];
     CK(cudaMemcpyAsync(hsq.data(), sq, sizeof(double) * np * ndet, cudaMemcpyDeviceToHost, st));
