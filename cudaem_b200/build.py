@@ -70,7 +70,7 @@ def build(force: bool = False, verbose: bool = False, ptxas_verbose: bool = Fals
         objs.append(obj)
         if force or _stale(obj, src, deps):
             cmd = [NVCC, "-ccbin", cxx, *ARCH, "-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr",
-                   "--split-compile=0", "-Xcompiler", "-fPIC,-ffp-contract=off", "-I", INCLUDE, "-c", src, "-o", obj]
+                   "-Xcompiler", "-fPIC,-ffp-contract=off", "-I", INCLUDE, "-c", src, "-o", obj]
             if ptxas_verbose:
                 cmd.insert(1, "-Xptxas=-v")
             jobs.append(cmd)
