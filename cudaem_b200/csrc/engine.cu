@@ -770,7 +770,11 @@ int l2_mode_for_waves(int nwaves, int64_t N)
 // launch latency between two steps shows, up to 2^19 wave pixels.  Per slice, plain and chained:
 // 1 x 256^2 6.74 and 5.84 us, 8 x 256^2 8.49 and 8.23, 1 x 512^2 11.56 and 10.54; but 1 x 1024^2
 // 15.9 and 16.4 (the next step's blocks land unevenly on the SMs), 64 x 1024^2 515 and 521.
-bool chain_steps(const ms_ctx* c, int nwaves, int64_t N) { return !c->profile && nwaves * N <= (1 << 19); }
+bool chain_steps(const ms_ctx* c, int nwaves, int64_t N)
+{
+    return !c->profile && nwaves * N <= (1 << 19) && c->stream != nullptr && c->stream != cudaStreamLegacy &&
+           c->stream != cudaStreamPerThread;
+}
 
 // Tile shape of the hot passes (row step on the transmission store, column step) for a batch of
 // nw waves on an nx x ny grid: forced by ms_set_tile_shape, else the fastest of the four
@@ -786,7 +790,8 @@ int choose_tile(ms_ctx* c, PassArgs pa, int nx, int ny, int nw, int nslices, cud
     if (c->tile_shape >= 0) return c->tile_shape;
     if ((!pa.tt && !pa.sV) || pa.variant == PASS_PIPELINED || nslices <= 0) return TILE_WIDE;
     char key[64];
-    std::snprintf(key, sizeof(key), "%d,%d,%d", nx, ny, nw);
+    // (2048-point steps on 32-thread teams, the gradient calls', are other kernels than the usual ones)
+    std::snprintf(key, sizeof(key), "%d,%d,%d%s", nx, ny, nw, (nx == 2048 || ny == 2048) && !pa.tw64 ? ",32" : "");
     auto it = c->tile_choice.find(key);
     if (it != c->tile_choice.end()) return it->second;
     if (c->profile) return TILE_WIDE;   // per-launch events would time the events
@@ -1168,6 +1173,8 @@ void sim_tem_like(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* o
         PassArgs pa = pass_args(s, psi, dwv, sVs, slot, cond);
         pa.l2_mode = l2_mode_for_waves(nw, N);
         pa.tt = sT;
+        pa.tile = choose_tile(c, pa, p.nx, p.ny, nw, g.S_cap, st);
+        c->last_tile = pa.tile;
         if (!force_cbed && p.simulation_type != MS_SIM_CBED) {
             // small batches take the short steps.  (CBED keeps the transforms it shares with an uneven
             // batch, so that a simulation gives the same values alone and in one; STEM keeps the
@@ -1175,8 +1182,6 @@ void sim_tem_like(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* o
             pa.short_x = s.short_x;
             pa.short_y = s.short_y;
         }
-        pa.tile = choose_tile(c, pa, p.nx, p.ny, nw, g.S_cap, st);
-        c->last_tile = pa.tile;
         if (iw == MS_IW_CONVERGENT) {
             pa.tw = s.tw_y;
             run_col(c, p.ny, COL_PROBE_INV, pa, nw, p.nx, st);
@@ -1767,8 +1772,9 @@ void sim_thickness(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* 
         float2* sT = (float2*)c->buf("sT", sizeof(float2) * slot * nw);
         run_potential(c, with_transmission(pot_args(p, s, A, g, nullptr, slot, 0, g.S_cap, 0), sT, s), nw, st);
         // filtered spectra of a chunk of slices, at most 256 MB (they are read back from L2 when they
-        // fit) or one slice
-        const int chunk = (int)std::max<int64_t>(1, std::min<int64_t>(nf, (256ll << 20) / (8 * N * nw)));
+        // fit) and a sixteenth of the free memory, or one slice
+        const int64_t room = std::min<int64_t>(256ll << 20, (int64_t)(c->free_mem() / 16));
+        const int chunk = (int)std::max<int64_t>(1, std::min<int64_t>(nf, room / (8 * N * nw)));
         // the waves' descriptors, then one per stored slice (only their weight is read)
         std::vector<WaveInfo> wv((size_t)nw + chunk);
         for (WaveInfo& w : wv) w.weight = (float)cs.weight;
@@ -1789,10 +1795,10 @@ void sim_thickness(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* 
         pa.aux_stride = (int64_t)chunk * N;
         pa.filt_g2in = g2in;
         pa.filt_g2out = g2out;
-        pa.short_x = s.short_x;
-        pa.short_y = s.short_y;
         pa.tile = choose_tile(c, pa, p.nx, p.ny, nw, g.S_cap, st);
         c->last_tile = pa.tile;
+        pa.short_x = s.short_x;
+        pa.short_y = s.short_y;
         const bool chain = chain_steps(c, nw, N);
         auto slices = [&] {
             PassArgs q = pa;
@@ -1875,6 +1881,17 @@ void sim_potential(ms_ctx* c, const ms_params& p, const ms_atoms& a, int conf, f
 // STEM on caller potentials (wave_modulation_batch, wave_function.cuh:74-87)
 // ---------------------------------------------------------------------------
 namespace {
+// A buffer the call can do without: null when the device has no room for it.
+void* optional_buf(ms_ctx* c, const char* name, size_t bytes)
+{
+    try {
+        return c->buf(name, bytes);
+    } catch (const MsError& e) {
+        if (e.st != MS_ERR_OUT_OF_MEMORY) throw;
+        return nullptr;
+    }
+}
+
 // The transmission t = exp(iV) of the caller's slices, formed once per call instead of once per
 // probe in the row steps (the same values), or null: with fewer than four probes the extra pass over
 // the slices costs what it saves, and the store may take a quarter of the free memory.  512^2, 16
@@ -1882,8 +1899,8 @@ namespace {
 float2* caller_transmission(ms_ctx* c, const Setup& s, const float* V, int64_t n, int np)
 {
     if (np < 4 || (double)n * sizeof(float2) > 0.25 * (double)c->free_mem()) return nullptr;
-    float2* T = (float2*)c->buf("caller_t", sizeof(float2) * n);
-    launch_transmission(V, n, s.exptab, T, c->stream);
+    float2* T = (float2*)optional_buf(c, "caller_t", sizeof(float2) * n);
+    if (T) launch_transmission(V, n, s.exptab, T, c->stream);
     return T;
 }
 }  // namespace
@@ -2026,8 +2043,11 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
     // The batch's launches replay from a graph when they hold none of the caller's pointers: on the
     // transmission store, with the gradient summed in the context's memory and copied out at the end
     // (where that takes at most a twentieth of the free memory).
-    const bool graphed = sT && (!on_dev || (double)slot * sizeof(float) <= 0.05 * (double)c->free_mem());
-    float* gV = on_dev && !graphed ? dV : (float*)c->buf("adj_dV", sizeof(float) * slot);
+    float* gV = !on_dev ? (float*)c->buf("adj_dV", sizeof(float) * slot) : nullptr;
+    if (on_dev && sT && (double)slot * sizeof(float) <= 0.05 * (double)c->free_mem())
+        gV = (float*)optional_buf(c, "adj_dV", sizeof(float) * slot);
+    const bool graphed = sT && gV;
+    if (!gV) gV = dV;
     float* gVw = (float*)c->buf("adj_dVw", sizeof(float) * N * B);   // per-wave planes of one slice
     double* partial = (double*)c->buf("det_part", sizeof(double) * B * nblk * ndet);
     double* Iw = (double*)c->buf("det_I", sizeof(double) * B * ndet);
