@@ -87,9 +87,9 @@ template <>
 struct ShortCfg<128> {
     static constexpr int T = 16, RA = 4, RB = 4;
 };
-// The batches they serve, in wave pixels: up to two waves of 512^2; shorter transforms have fewer
-// points per thread to begin with, and lose from 2^18 pixels on (figures in fft.cuh)
-inline bool short_step(int N, long long pixels) { return N <= 512 && pixels <= (N == 512 ? 1 << 19 : 1 << 17); }
+// The batches they serve, in wave pixels: up to two waves of 512^2 (four lose), four of 256^2 (6.75 ->
+// 6.48 us per slice; eight 8.6 -> 9.3), sixteen of 128^2 (7.3 -> 6.3; thirty-two 8.0 -> 8.6)
+inline bool short_step(int N, long long pixels) { return N <= 512 && pixels <= (N == 512 ? 1 << 19 : 1 << 18); }
 
 template <int N, int ROWS_ = FftCfg<N>::ROWS, int TC_ = FftCfg<N>::TC>
 struct FftLayoutT {
