@@ -142,7 +142,7 @@ struct EngineArgs {
 // Kernel form of ROW_INV_T_FWD and COL_STEP.  PASS_CLASSIC (the default) launches the classic
 // one-block-per-tile kernels slice by slice for CBED / TEM / STEM (measured fastest there) and runs
 // an uneven batch's grid groups in the persistent slice engine (measured 1.35x faster there, with
-// half the completion latency); PASS_PIPELINED the persistent pipelined kernels (grids of
+// half the completion latency; groups of 2048 points slice by slice, see k_row_2048); PASS_PIPELINED the persistent pipelined kernels (grids of
 // 128..1024 points); PASS_ENGINE the slice engine everywhere; PASS_PER_SLICE the classic kernels
 // everywhere.  All compute the same operations.
 enum PassVariant { PASS_CLASSIC = 0, PASS_PIPELINED = 1, PASS_ENGINE = 2, PASS_PER_SLICE = 3 };

@@ -206,8 +206,8 @@ int ms_last_probe_batch(const ms_ctx* ctx);
 ms_status ms_set_graphs(ms_ctx* ctx, int enable);
 /* Kernel form of the hot slice passes: 0 (default) the classic kernels, one block per tile
  * of rows or columns, launched slice by slice for CBED / TEM / STEM, while an uneven batch's grid
- * groups run in the persistent slice engine (form 2); 3 the classic kernels everywhere, uneven
- * batches included; 1 the persistent pipelined kernels
+ * groups run in the persistent slice engine (form 2; groups of 2048 points slice by slice); 3 the
+ * classic kernels everywhere, uneven batches included; 1 the persistent pipelined kernels
  * (one block per SM walking the work items, the next item's wave prefetched while the
  * current one is transformed) for grids of 128..1024 points per axis; 2 the persistent slice
  * engine: on square grids, every slice of a CBED / TEM / STEM batch or of an uneven batch's
