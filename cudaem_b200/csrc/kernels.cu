@@ -326,7 +326,7 @@ size_t col_smem(int N)
 
 // ---------------------------------------------------------------------------
 // projected potential: gen_slice_potential_kernel (device_kernels.cuh:28-47)
-// restructured as atom-culled 64x16 pixel tiles with float4 stores
+// restructured as atom-culled 64x32 pixel tiles, walked in slots of 8x4 pixels
 // ---------------------------------------------------------------------------
 constexpr int kPotTX = 64, kPotTY = 32, kPotThreads = 256;
 constexpr int kPotBlocks = 8;   // per SM; 6 and 5 blocks (40, 48 registers) were slower: 8.5 and 9.1 against 8.1 ms below
