@@ -1386,7 +1386,8 @@ int autotune_batch(ms_ctx* c, const ms_params& p, const Setup& s, const PassArgs
     for (int b = 32; b <= 256; b *= 2)
         if (b <= hi) cand.push_back(b);
     if (cand.empty()) return std::max(1, hi);
-    if (cand.size() == 1 || c->profile) return cand.back();
+    // (the timed row steps read the slices: without a store there is nothing to time)
+    if (cand.size() == 1 || c->profile || (!base.tt && !base.sV)) return cand.back();
     char key[96];
     std::snprintf(key, sizeof(key), "%d,%d,%d,%d", p.nx, p.ny, std::min(S, 2), hi);
     auto it = c->batch_choice.find(key);
@@ -1643,7 +1644,7 @@ void sim_stem(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* out)
         WaveInfo* dwv_all = (WaveInfo*)c->buf("waves_all", sizeof(WaveInfo) * npos);
         upload(c, dwv_all, wv.data(), sizeof(WaveInfo) * npos, st);
         if (!tuned) {
-            PassArgs base = pass_args(s, nullptr, nullptr, nullptr, slot, cond);
+            PassArgs base = pass_args(s, nullptr, nullptr, sVs, slot, cond);   // on the store in use
             base.tt = sT;
             B = autotune_batch(c, p, s, base, wv[0], S, npos, cap);
             tuned = true;
