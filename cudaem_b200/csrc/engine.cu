@@ -1853,6 +1853,20 @@ void sim_thickness(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* 
 // ---------------------------------------------------------------------------
 // projected potentials of one configuration
 // ---------------------------------------------------------------------------
+// Whether a kernel may store floats through a caller's pointer: aligned memory of the context's device.
+// Anything else that a copy takes (another GPU's memory, a pointer inside a packed record) is written by
+// a copy.
+static bool kernel_can_store(const ms_ctx* c, const void* p)
+{
+    if ((uintptr_t)p % alignof(float) != 0) return false;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeDevice && at.device == c->device;
+}
+
 void sim_potential(ms_ctx* c, const ms_params& p, const ms_atoms& a, int conf, float* V, int64_t cap, int on_dev,
                    int* n_slices)
 {
@@ -1870,10 +1884,11 @@ void sim_potential(ms_ctx* c, const ms_params& p, const ms_atoms& a, int conf, f
     if (V) {
         MS_REQUIRE((int64_t)S * s.N <= cap, MS_ERR_INVALID_ARG, "V_out holds fewer than n_slices*ny*nx floats");
         int64_t slot = (int64_t)S * s.N;
-        // straight into a device buffer of the caller's (the kernel stores single floats)
-        float* sV = on_dev ? V : (float*)c->buf("sV", sizeof(float) * slot);
+        // straight into a device buffer of the caller's where the kernel can store there
+        const bool direct = on_dev && kernel_can_store(c, V);
+        float* sV = direct ? V : (float*)c->buf("sV", sizeof(float) * slot);
         run_potential(c, pot_args(p, s, A, g, sV, slot, 0, S, 0), 1, st);
-        if (!on_dev) copy_out(c, V, sV, slot, 0);
+        if (!direct) copy_out(c, V, sV, slot, on_dev);
     }
     tm.stop();
 }
