@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <initializer_list>
 #include <map>
 #include <string>
 #include <vector>
@@ -33,6 +34,8 @@ struct ms_ctx {
     struct Buf {
         void* p = nullptr;
         size_t bytes = 0;
+        bool spare = false;   // the calls can do without it (spare_buf)
+        bool lent = false;    // a spare one that the running call uses
     };
     std::map<std::string, Buf> bufs;             // device buffers reused across calls
     std::map<int, void*> twiddles;               // inter-level FFT twiddles per transform length
@@ -73,10 +76,19 @@ struct ms_ctx {
     // A device buffer of at least `bytes`, kept for later calls.  Growing a buffer first
     // drains the stream so that no queued kernel still reads the old allocation.
     void* buf(const std::string& name, size_t bytes);
+    // A buffer that only makes a call faster: null when the device has no room for it.  It stays for later
+    // calls, but the calls that do not use it count it as free memory, and it is given back as soon
+    // as one of them needs the room.  Take it after the buffers the call cannot do without.
+    void* spare_buf(const std::string& name, size_t bytes);
+    void return_spares();   // a call begins: none is in use
+    bool drop_spares();     // frees those not in use; false: there were none
+    // Bytes that free_mem() does not count, held under these names by earlier calls: a size chosen by
+    // free_mem() + held() is the same on every call.
+    size_t held(std::initializer_list<const char*> names) const;
     void release_all();
 
-    // Free device memory as cudaMemGetInfo reports it.  The reading is kept until this context
-    // allocates or frees device memory: the query is a driver call that can wait behind other
+    // Free device memory as cudaMemGetInfo reports it, and the spare buffers that are not in use.  The
+    // reading is kept until this context allocates or frees device memory: the query is a driver call that can wait behind other
     // processes' queries of the device (a monitoring tool polling clocks, for one), and every
     // simulation asks for it at its start, while the GPU is idle.
     size_t free_mem();

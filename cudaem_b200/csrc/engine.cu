@@ -39,12 +39,16 @@ size_t ms_ctx::free_mem()
         free_seen = fr;
         free_known = true;
     }
-    return free_seen;
+    size_t spare = 0;
+    for (const auto& kv : bufs)
+        if (kv.second.spare && !kv.second.lent) spare += kv.second.bytes;
+    return free_seen + spare;
 }
 
 void* ms_ctx::buf(const std::string& name, size_t bytes)
 {
     Buf& b = bufs[name];
+    b.lent = true;
     if (b.p && b.bytes >= bytes) return b.p;
     forget_free_mem();
     if (b.p) {
@@ -56,7 +60,12 @@ void* ms_ctx::buf(const std::string& name, size_t bytes)
     }
     size_t want = std::max<size_t>(bytes, 256);
     void* p = nullptr;
-    cudaError_t e = inject == MS_INJECT_ALLOC_FAIL ? cudaErrorMemoryAllocation : cudaMalloc(&p, want);
+    auto alloc = [&] { return inject == MS_INJECT_ALLOC_FAIL ? cudaErrorMemoryAllocation : cudaMalloc(&p, want); };
+    cudaError_t e = alloc();
+    if (e == cudaErrorMemoryAllocation && drop_spares()) {
+        cudaGetLastError();
+        e = alloc();
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         throw msb::MsError(MS_ERR_OUT_OF_MEMORY,
@@ -65,6 +74,52 @@ void* ms_ctx::buf(const std::string& name, size_t bytes)
     b.p = p;
     b.bytes = want;
     return p;
+}
+
+void* ms_ctx::spare_buf(const std::string& name, size_t bytes)
+{
+    void* p = nullptr;
+    try {
+        p = buf(name, bytes);
+    } catch (const msb::MsError& e) {
+        if (e.st != MS_ERR_OUT_OF_MEMORY) throw;
+    }
+    bufs[name].spare = true;
+    return p;
+}
+
+void ms_ctx::return_spares()
+{
+    for (auto& kv : bufs) kv.second.lent = false;
+}
+
+bool ms_ctx::drop_spares()
+{
+    bool freed = false;
+    for (auto& kv : bufs) {
+        Buf& b = kv.second;
+        if (!b.spare || b.lent || !b.p) continue;
+        if (!freed) {
+            cudaStreamSynchronize(stream);
+            drop_graph();   // a captured graph may hold the address
+        }
+        cudaFree(b.p);
+        b.p = nullptr;
+        b.bytes = 0;
+        freed = true;
+    }
+    if (freed) forget_free_mem();
+    return freed;
+}
+
+size_t ms_ctx::held(std::initializer_list<const char*> names) const
+{
+    size_t sum = 0;
+    for (const char* n : names) {
+        auto it = bufs.find(n);
+        if (it != bufs.end() && !(it->second.spare && !it->second.lent)) sum += it->second.bytes;
+    }
+    return sum;
 }
 
 void* ms_ctx::stage_take(size_t bytes)
@@ -967,6 +1022,7 @@ struct Timer {
         if (c->stage_busy) CK(cudaDeviceSynchronize());
         c->stage_off = ms_ctx::kStageFirst;
         c->stage_busy = true;
+        c->return_spares();
         CK(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
         CK(cudaEventRecord(c->ev0, c->stream));
     }
@@ -1764,7 +1820,8 @@ void sim_thickness(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* 
     // (256^2, 24 slices, 2 configurations: 1697 us per call before, 875 us so, 746 us with short chained steps).
     const size_t per_conf = (size_t)estimate_slices(p, a) * N * 8 + (size_t)N * 8 * 2 + (size_t)a.n * 40 +
                             fine_bytes_per_conf(p, a);
-    const int gsize = (int)std::max<size_t>(1, std::min<size_t>(cs.confs.size(), free_budget(c) / per_conf));
+    const size_t budget = (size_t)(0.6 * (double)(c->free_mem() + c->held({"sT", "psi", "thick_aux"})));
+    const int gsize = (int)std::max<size_t>(1, std::min<size_t>(cs.confs.size(), budget / per_conf));
     for (size_t g0 = 0; g0 < cs.confs.size(); g0 += gsize) {
         const std::vector<int> confs(cs.confs.begin() + g0, cs.confs.begin() + std::min(cs.confs.size(), g0 + gsize));
         SpecGroup g = build_specimen(c, p, A, confs, s.ph);
@@ -1774,7 +1831,7 @@ void sim_thickness(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* 
         run_potential(c, with_transmission(pot_args(p, s, A, g, nullptr, slot, 0, g.S_cap, 0), sT, s), nw, st);
         // filtered spectra of a chunk of slices, at most 256 MB (they are read back from L2 when they
         // fit) and a sixteenth of the free memory, or one slice
-        const int64_t room = std::min<int64_t>(256ll << 20, (int64_t)(c->free_mem() / 16));
+        const int64_t room = std::min<int64_t>(256ll << 20, (int64_t)((c->free_mem() + c->held({"psi", "thick_aux"})) / 16));
         const int chunk = (int)std::max<int64_t>(1, std::min<int64_t>(nf, room / (8 * N * nw)));
         // the waves' descriptors, then one per stored slice (only their weight is read)
         std::vector<WaveInfo> wv((size_t)nw + chunk);
@@ -1897,25 +1954,14 @@ void sim_potential(ms_ctx* c, const ms_params& p, const ms_atoms& a, int conf, f
 // STEM on caller potentials (wave_modulation_batch, wave_function.cuh:74-87)
 // ---------------------------------------------------------------------------
 namespace {
-// A buffer the call can do without: null when the device has no room for it.
-void* optional_buf(ms_ctx* c, const char* name, size_t bytes)
-{
-    try {
-        return c->buf(name, bytes);
-    } catch (const MsError& e) {
-        if (e.st != MS_ERR_OUT_OF_MEMORY) throw;
-        return nullptr;
-    }
-}
-
 // The transmission t = exp(iV) of the caller's slices, formed once per call instead of once per
 // probe in the row steps (the same values), or null: with fewer than four probes the extra pass over
-// the slices costs what it saves, and the store may take a quarter of the free memory.  512^2, 16
-// probes: the row step takes 15 us on the store and 25 us on V.
+// the slices costs what it saves, and the store may take a quarter of the memory that the call's own
+// buffers leave.  512^2, 16 probes: the row step takes 15 us on the store and 25 us on V.
 float2* caller_transmission(ms_ctx* c, const Setup& s, const float* V, int64_t n, int np)
 {
     if (np < 4 || (double)n * sizeof(float2) > 0.25 * (double)c->free_mem()) return nullptr;
-    float2* T = (float2*)optional_buf(c, "caller_t", sizeof(float2) * n);
+    float2* T = (float2*)c->spare_buf("caller_t", sizeof(float2) * n);
     if (T) launch_transmission(V, n, s.exptab, T, c->stream);
     return T;
 }
@@ -1946,11 +1992,14 @@ void sim_stem_forward_potential(ms_ctx* c, const ms_params& p, const float* V, i
     }
     float* dthr = (float*)c->buf("det_thr", sizeof(float) * 2 * ndet);
     upload(c, dthr, thr.data(), sizeof(float) * 2 * ndet, st);
-    float2* sT = caller_transmission(c, s, sV, slot, np);
     const int B = std::min(np, p.probe_batch > 0 ? p.probe_batch : 256);
     const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>(64, N / 4096));
     double* partial = (double*)c->buf("det_part", sizeof(double) * B * nblk * ndet);
     double* Iw = (double*)c->buf("det_I_all", sizeof(double) * np * ndet);
+    float* o = (float*)c->buf("stem_out", sizeof(float) * np * ndet);
+    WaveInfo* dwv = (WaveInfo*)c->buf("waves", sizeof(WaveInfo) * B);
+    float2* psi = (float2*)c->buf("psi", sizeof(float2) * N * B);
+    float2* sT = caller_transmission(c, s, sV, slot, np);
     const double cc10 = gate_coef(-kPi * (p.cond_lens.c10 + z_init) * s.ph.lambda);
     std::vector<WaveInfo> wv((size_t)B);
     for (int start = 0; start < np; start += B) {
@@ -1964,9 +2013,7 @@ void sim_stem_forward_potential(ms_ctx* c, const ms_params& p, const float* V, i
             wv[i].weight = 1.0f;
             wv[i].pos = start + i;
         }
-        WaveInfo* dwv = (WaveInfo*)c->buf("waves", sizeof(WaveInfo) * B);
         upload(c, dwv, wv.data(), sizeof(WaveInfo) * nb, st);
-        float2* psi = (float2*)c->buf("psi", sizeof(float2) * N * B);
         PassArgs pa = pass_args(s, psi, dwv, sV, slot, cond);
         pa.tt = sT;
         // the tile shape is tuned as for the simulations, and the waves stay in L2 where they fit
@@ -1995,7 +2042,6 @@ void sim_stem_forward_potential(ms_ctx* c, const ms_params& p, const float* V, i
         else body();
         CK(cudaStreamSynchronize(st));
     }
-    float* o = (float*)c->buf("stem_out", sizeof(float) * np * ndet);
     launch_d2f(Iw, (int64_t)np * ndet, o, st);
     CK(cudaMemcpyAsync(I, o, sizeof(float) * np * ndet, cudaMemcpyDeviceToHost, st));
     tm.stop();
@@ -2041,14 +2087,14 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
     float* dtgt = (float*)c->buf("adj_target", sizeof(float) * np * ndet);
     upload(c, dtgt, target, sizeof(float) * np * ndet, st);
 
-    float2* sT = caller_transmission(c, s, sV, slot, np);
     const int k = p.ckpt_interval;
     const int nseg = (S + k - 1) / k;
     // probes per batch: adjoint wave, forward wave, one segment of transmitted waves and the
     // checkpoints must fit the memory budget
     const size_t per_wave = (size_t)N * 8 * (2 + 2 * (size_t)k + (size_t)(nseg - 1)) + (size_t)N * 4;
     int B = p.probe_batch > 0 ? p.probe_batch : 256;
-    B = (int)std::max<size_t>(1, std::min<size_t>((size_t)B, free_budget(c) / per_wave));
+    const size_t room = c->free_mem() + c->held({"adj_psi", "adj_xseg", "adj_ckpt", "adj_dVw", "adj_dV"});
+    B = (int)std::max<size_t>(1, std::min<size_t>((size_t)B, (size_t)(0.6 * (double)room) / per_wave));
     B = std::min(B, np);
     const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>(64, N / 4096));
     const int tiles = col_tiles(p.ny, p.nx);
@@ -2056,14 +2102,6 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
     // transmitted waves of two segments: the one being swept back and the one being recomputed
     float2* xseg = (float2*)c->buf("adj_xseg", sizeof(float2) * N * B * k * 2);
     float2* ckpt = nseg > 1 ? (float2*)c->buf("adj_ckpt", sizeof(float2) * N * B * (nseg - 1)) : nullptr;
-    // The batch's launches replay from a graph when they hold none of the caller's pointers: on the
-    // transmission store, with the gradient summed in the context's memory and copied out at the end
-    // (where that takes at most a twentieth of the free memory).
-    float* gV = !on_dev ? (float*)c->buf("adj_dV", sizeof(float) * slot) : nullptr;
-    if (on_dev && sT && (double)slot * sizeof(float) <= 0.05 * (double)c->free_mem())
-        gV = (float*)optional_buf(c, "adj_dV", sizeof(float) * slot);
-    const bool graphed = sT && gV;
-    if (!gV) gV = dV;
     float* gVw = (float*)c->buf("adj_dVw", sizeof(float) * N * B);   // per-wave planes of one slice
     double* partial = (double*)c->buf("det_part", sizeof(double) * B * nblk * ndet);
     double* Iw = (double*)c->buf("det_I", sizeof(double) * B * ndet);
@@ -2071,6 +2109,16 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
     double* sq = (double*)c->buf("adj_sq", sizeof(double) * np * ndet);
     double* chi_part = (double*)c->buf("adj_chi_part", sizeof(double) * B * tiles * 2);
     double* chi_acc = (double*)c->buf("adj_chi", sizeof(double) * 2);
+    WaveInfo* dwv = (WaveInfo*)c->buf("waves", sizeof(WaveInfo) * B);
+    float* gV = !on_dev ? (float*)c->buf("adj_dV", sizeof(float) * slot) : nullptr;
+    float2* sT = caller_transmission(c, s, sV, slot, np);
+    // The batch's launches replay from a graph when they hold none of the caller's pointers: on the
+    // transmission store, with the gradient summed in the context's memory and copied out at the end
+    // (where that takes at most a twentieth of the free memory).
+    if (on_dev && sT && (double)slot * sizeof(float) <= 0.05 * (double)c->free_mem())
+        gV = (float*)c->spare_buf("adj_dV", sizeof(float) * slot);
+    const bool graphed = sT && gV;
+    if (!gV) gV = dV;
     CK(cudaMemsetAsync(gV, 0, sizeof(float) * slot, st));
     CK(cudaMemsetAsync(chi_acc, 0, sizeof(double) * 2, st));
     const double cc10 = gate_coef(-kPi * (p.cond_lens.c10 + z_init) * s.ph.lambda);
@@ -2087,7 +2135,6 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
             wv[i].weight = 1.0f;
             wv[i].pos = start + i;
         }
-        WaveInfo* dwv = (WaveInfo*)c->buf("waves", sizeof(WaveInfo) * B);
         upload(c, dwv, wv.data(), sizeof(WaveInfo) * nb, st);
         PassArgs pa = pass_args(s, adj, dwv, sV, slot, cond);
         pa.tt = sT;
