@@ -80,6 +80,7 @@ struct ms_ctx {
     // calls, but the calls that do not use it count it as free memory, and it is given back as soon
     // as one of them needs the room.  Take it after the buffers the call cannot do without.
     void* spare_buf(const std::string& name, size_t bytes);
+    bool has(const std::string& name, size_t bytes) const;   // held already, at this size or larger
     void return_spares();   // a call begins: none is in use
     bool drop_spares();     // frees those not in use; false: there were none
     // Bytes that free_mem() does not count, held under these names by earlier calls: a size chosen by

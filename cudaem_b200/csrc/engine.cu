@@ -88,6 +88,12 @@ void* ms_ctx::spare_buf(const std::string& name, size_t bytes)
     return p;
 }
 
+bool ms_ctx::has(const std::string& name, size_t bytes) const
+{
+    auto it = bufs.find(name);
+    return it != bufs.end() && it->second.p && it->second.bytes >= bytes;
+}
+
 void ms_ctx::return_spares()
 {
     for (auto& kv : bufs) kv.second.lent = false;
@@ -1957,11 +1963,13 @@ namespace {
 // The transmission t = exp(iV) of the caller's slices, formed once per call instead of once per
 // probe in the row steps (the same values), or null: with fewer than four probes the extra pass over
 // the slices costs what it saves, and the store may take a quarter of the memory that the call's own
-// buffers leave.  512^2, 16 probes: the row step takes 15 us on the store and 25 us on V.
+// buffers leave (or what an earlier call left it).  512^2, 16 probes: the row step takes 15 us on the store
+// and 25 us on V.
 float2* caller_transmission(ms_ctx* c, const Setup& s, const float* V, int64_t n, int np)
 {
-    if (np < 4 || (double)n * sizeof(float2) > 0.25 * (double)c->free_mem()) return nullptr;
-    float2* T = (float2*)c->spare_buf("caller_t", sizeof(float2) * n);
+    const size_t bytes = sizeof(float2) * n;
+    if (np < 4 || !(c->has("caller_t", bytes) || (double)bytes <= 0.25 * (double)c->free_mem())) return nullptr;
+    float2* T = (float2*)c->spare_buf("caller_t", bytes);
     if (T) launch_transmission(V, n, s.exptab, T, c->stream);
     return T;
 }
@@ -2114,8 +2122,9 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
     float2* sT = caller_transmission(c, s, sV, slot, np);
     // The batch's launches replay from a graph when they hold none of the caller's pointers: on the
     // transmission store, with the gradient summed in the context's memory and copied out at the end
-    // (where that takes at most a twentieth of the free memory).
-    if (on_dev && sT && (double)slot * sizeof(float) <= 0.05 * (double)c->free_mem())
+    // (where that takes at most a twentieth of the free memory, or is held already).
+    if (on_dev && sT &&
+        (c->has("adj_dV", sizeof(float) * slot) || (double)slot * sizeof(float) <= 0.05 * (double)c->free_mem()))
         gV = (float*)c->spare_buf("adj_dV", sizeof(float) * slot);
     const bool graphed = sT && gV;
     if (!gV) gV = dV;
