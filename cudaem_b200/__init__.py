@@ -259,6 +259,10 @@ class Context:
     def last_probe_batch(self) -> int:
         return lib().ms_last_probe_batch(self.handle)
 
+    @property
+    def last_graph_captures(self) -> int:
+        return lib().ms_last_graph_captures(self.handle)
+
     def set_graphs(self, enable: bool) -> None:
         self.check(lib().ms_set_graphs(self.handle, 1 if enable else 0))
 

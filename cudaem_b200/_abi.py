@@ -152,6 +152,7 @@ PROTOTYPES = {
                                    _P(C.c_double), C.c_int, _P(C.c_float), _P(C.c_double), _P(C.c_float),
                                    _P(C.c_double), _P(C.c_double)]),
     "ms_last_probe_batch": (C.c_int, [C.c_void_p]),
+    "ms_last_graph_captures": (C.c_int, [C.c_void_p]),
     "ms_set_graphs": (C.c_int, [C.c_void_p, C.c_int]),
     "ms_set_pass_kernels": (C.c_int, [C.c_void_p, C.c_int]),
     "ms_set_tile_shape": (C.c_int, [C.c_void_p, C.c_int]),

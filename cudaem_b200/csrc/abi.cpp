@@ -166,6 +166,7 @@ double ms_last_device_ms(const ms_ctx* c) { return c ? c->last_ms : 0.0; }
 int64_t ms_last_launch_count(const ms_ctx* c) { return c ? c->last_launches : 0; }
 
 int ms_last_probe_batch(const ms_ctx* c) { return c ? c->last_batch : 0; }
+int ms_last_graph_captures(const ms_ctx* c) { return c ? c->last_captures : 0; }
 
 ms_status ms_set_pass_kernels(ms_ctx* c, int variant)
 {

@@ -46,8 +46,12 @@ struct ms_ctx {
     struct Graph {
         cudaGraphExec_t exec = nullptr;
         int64_t launches = 0;                    // kernels inside the captured graph
+        uint64_t used = 0;                       // graph_clock at its last replay
     };
-    std::map<std::string, Graph> graphs;         // keyed by the launch arguments they bake in
+    std::map<std::string, Graph> graphs;         // keyed by the launch arguments they bake in; at most kMaxGraphs
+    static constexpr size_t kMaxGraphs = 8;      // the full and the last batch of four kinds of call
+    uint64_t graph_clock = 0;
+    int last_captures = 0;                       // graphs captured by the last call
     bool use_graphs = true;
     int pass_variant = 0;                        // msb::PassVariant of the slice-pass kernels (0: classic)
     bool pot_overlap = false;                    // potential chunks on a side stream beside the slice passes

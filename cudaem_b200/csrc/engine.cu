@@ -1028,6 +1028,7 @@ struct Timer {
         if (c->stage_busy) CK(cudaDeviceSynchronize());
         c->stage_off = ms_ctx::kStageFirst;
         c->stage_busy = true;
+        c->last_captures = 0;
         c->return_spares();
         CK(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
         CK(cudaEventRecord(c->ev0, c->stream));
@@ -1133,7 +1134,13 @@ void run_graphed(ms_ctx* c, const std::string& key, F&& body)
     }
     auto it = c->graphs.find(key);
     if (it == c->graphs.end()) {
-        if (c->graphs.size() >= 4) c->drop_graph();   // full batches, the last partial batch, ...
+        if (c->graphs.size() >= ms_ctx::kMaxGraphs) {
+            auto old = c->graphs.begin();
+            for (auto g = c->graphs.begin(); g != c->graphs.end(); ++g)
+                if (g->second.used < old->second.used) old = g;
+            cudaGraphExecDestroy(old->second.exec);
+            c->graphs.erase(old);
+        }
         const int64_t l0 = kernel_launches();
         CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         try {
@@ -1156,7 +1163,9 @@ void run_graphed(ms_ctx* c, const std::string& key, F&& body)
         gr.launches = kernel_launches() - l0;
         add_kernel_launches(-gr.launches);   // captured, not run
         it = c->graphs.emplace(key, gr).first;
+        c->last_captures++;
     }
+    it->second.used = ++c->graph_clock;
     CK(cudaGraphLaunch(it->second.exec, st));
     add_kernel_launches(it->second.launches);
 }
@@ -1864,12 +1873,14 @@ void sim_thickness(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* 
         pa.short_x = s.short_x;
         pa.short_y = s.short_y;
         const bool chain = chain_steps(c, nw, N);
+        if (iw == MS_IW_CONVERGENT) {
+            PassArgs q = pa;
+            q.tw = s.tw_y;
+            run_col(c, p.ny, COL_PROBE_INV, q, nw, p.nx, st);
+        }
+        std::memset(&pa.lens, 0, sizeof(pa.lens));   // the probe alone reads it: the loop's graph serves every lens
         auto slices = [&] {
             PassArgs q = pa;
-            if (iw == MS_IW_CONVERGENT) {
-                q.tw = s.tw_y;
-                run_col(c, p.ny, COL_PROBE_INV, q, nw, p.nx, st);
-            }
             for (int s0 = 0; s0 < nf; s0 += chunk) {
                 const int s1 = std::min(nf, s0 + chunk);
                 for (int sl = s0; sl < s1; sl++) {
@@ -2003,7 +2014,7 @@ void sim_stem_forward_potential(ms_ctx* c, const ms_params& p, const float* V, i
     const int B = std::min(np, p.probe_batch > 0 ? p.probe_batch : 256);
     const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>(64, N / 4096));
     double* partial = (double*)c->buf("det_part", sizeof(double) * B * nblk * ndet);
-    double* Iw = (double*)c->buf("det_I_all", sizeof(double) * np * ndet);
+    double* Iw = (double*)c->buf("det_I", sizeof(double) * B * ndet);
     float* o = (float*)c->buf("stem_out", sizeof(float) * np * ndet);
     WaveInfo* dwv = (WaveInfo*)c->buf("waves", sizeof(WaveInfo) * B);
     float2* psi = (float2*)c->buf("psi", sizeof(float2) * N * B);
@@ -2027,30 +2038,33 @@ void sim_stem_forward_potential(ms_ctx* c, const ms_params& p, const float* V, i
         // the tile shape is tuned as for the simulations, and the waves stay in L2 where they fit
         pa.l2_mode = l2_mode_for_waves(nb, N);
         pa.tile = choose_tile(c, pa, p.nx, p.ny, nb, S, st);
-        // on the transmission store the launches hold none of the caller's pointers, so the loop replays
-        // from a graph whatever buffers the next call brings
+        pa.tw = s.tw_y;
+        run_col(c, p.ny, COL_PROBE_INV, pa, nb, p.nx, st);
+        // on the transmission store the launches hold none of the caller's pointers, nothing of the lens and
+        // nothing that tells one full batch from the next, so the loop replays from one graph for all
+        // of them whatever the next call brings
         if (sT) pa.sV = nullptr;
-        double* Ib = Iw + (int64_t)start * ndet;
+        std::memset(&pa.lens, 0, sizeof(pa.lens));
+        const bool chain = chain_steps(c, nb, N);
         auto body = [&] {
             PassArgs q = pa;
-            q.tw = s.tw_y;
-            run_col(c, p.ny, COL_PROBE_INV, q, nb, p.nx, st);
-            q.chained = chain_steps(c, nb, N);
             for (int sl = 0; sl < S; sl++) {
                 q.slice = sl;
+                q.chained = chain && sl > 0;
                 q.tw = s.tw_x;
                 run_row(c, p.nx, ROW_INV_T_FWD, q, nb, p.ny, st);
+                q.chained = chain;
                 q.tw = s.tw_y;
                 run_col(c, p.ny, COL_STEP, q, nb, p.nx, st);
             }
             launch_detect(psi, nb, p.nx, p.ny, s.gd.dgx_f, s.gd.dgy_f, dthr, dthr + ndet, ndet, partial, nblk, st);
-            launch_det_finalize(partial, nb, nblk, ndet, dwv, Ib, nullptr, 0, 0, st);
+            launch_det_finalize(partial, nb, nblk, ndet, dwv, Iw, nullptr, 0, 0, st);
         };
-        if (sT) run_graphed(c, graph_key_of(pa, nb, S, nblk, ndet, partial, Ib, nullptr, dthr, -3), body);
+        if (sT) run_graphed(c, graph_key_of(pa, nb, S, nblk, ndet, partial, Iw, nullptr, dthr, -3), body);
         else body();
+        launch_d2f(Iw, (int64_t)nb * ndet, o + (int64_t)start * ndet, st);
         CK(cudaStreamSynchronize(st));
     }
-    launch_d2f(Iw, (int64_t)np * ndet, o, st);
     CK(cudaMemcpyAsync(I, o, sizeof(float) * np * ndet, cudaMemcpyDeviceToHost, st));
     tm.stop();
 }
@@ -2092,9 +2106,6 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
     }
     float* dthr = (float*)c->buf("det_thr", sizeof(float) * 2 * ndet);
     upload(c, dthr, thr.data(), sizeof(float) * 2 * ndet, st);
-    float* dtgt = (float*)c->buf("adj_target", sizeof(float) * np * ndet);
-    upload(c, dtgt, target, sizeof(float) * np * ndet, st);
-
     const int k = p.ckpt_interval;
     const int nseg = (S + k - 1) / k;
     // probes per batch: adjoint wave, forward wave, one segment of transmitted waves and the
@@ -2114,7 +2125,8 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
     double* partial = (double*)c->buf("det_part", sizeof(double) * B * nblk * ndet);
     double* Iw = (double*)c->buf("det_I", sizeof(double) * B * ndet);
     double* resid = (double*)c->buf("adj_resid", sizeof(double) * B * ndet);
-    double* sq = (double*)c->buf("adj_sq", sizeof(double) * np * ndet);
+    double* sq = (double*)c->buf("adj_sq", sizeof(double) * B * ndet);
+    float* dtgt = (float*)c->buf("adj_target", sizeof(float) * B * ndet);
     double* chi_part = (double*)c->buf("adj_chi_part", sizeof(double) * B * tiles * 2);
     double* chi_acc = (double*)c->buf("adj_chi", sizeof(double) * 2);
     WaveInfo* dwv = (WaveInfo*)c->buf("waves", sizeof(WaveInfo) * B);
@@ -2132,6 +2144,7 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
     CK(cudaMemsetAsync(chi_acc, 0, sizeof(double) * 2, st));
     const double cc10 = gate_coef(-kPi * (p.cond_lens.c10 + z_init) * s.ph.lambda);
     std::vector<WaveInfo> wv((size_t)B);
+    std::vector<double> hsq((size_t)np * ndet);
     for (int start = 0; start < np; start += B) {
         const int nb = std::min(B, np - start);
         const int64_t wstride = (int64_t)nb * N;   // one slice of the batch in xseg / ckpt
@@ -2145,6 +2158,7 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
             wv[i].pos = start + i;
         }
         upload(c, dwv, wv.data(), sizeof(WaveInfo) * nb, st);
+        upload(c, dtgt, target + (int64_t)start * ndet, sizeof(float) * nb * ndet, st);
         PassArgs pa = pass_args(s, adj, dwv, sV, slot, cond);
         pa.tt = sT;
         // forward, recomputed and adjoint steps are those whose transforms the adjoint kernels share
@@ -2155,13 +2169,17 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
         pa.ndet = ndet;
         pa.resid = resid;
         pa.chi_part = chi_part;
+        // the probe and its gradient alone read the lens; without them (and the caller's pointers) one
+        // graph serves every full batch of every call
+        PassArgs probe = pa;
+        probe.tw = s.tw_y;
+        run_col(c, p.ny, COL_PROBE_INV, probe, nb, p.nx, st);
         if (graphed) pa.sV = nullptr;
+        std::memset(&pa.lens, 0, sizeof(pa.lens));
         const PassArgs pa0 = pa;
         auto body = [&] {
             PassArgs pa = pa0;
             // forward sweep with checkpoints
-            pa.tw = s.tw_y;
-            run_col(c, p.ny, COL_PROBE_INV, pa, nb, p.nx, st);
             const int last0 = (nseg - 1) * k;
             auto xbuf = [&](int seg) { return xseg + (int64_t)(seg % 2) * k * wstride; };
             for (int sl = 0; sl < S; sl++) {
@@ -2179,7 +2197,7 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
             }
             launch_detect(adj, nb, p.nx, p.ny, s.gd.dgx_f, s.gd.dgy_f, dthr, dthr + ndet, ndet, partial, nblk, st);
             launch_det_finalize(partial, nb, nblk, ndet, dwv, Iw, nullptr, 0, 0, st);
-            launch_resid(Iw, dtgt + (int64_t)start * ndet, nb * ndet, resid, sq + (int64_t)start * ndet, st);
+            launch_resid(Iw, dtgt, nb * ndet, resid, sq, st);
             pa.tw = s.tw_y;
             run_col(c, p.ny, COL_SEED, pa, nb, p.nx, st);
             // Segments are recomputed on a second stream one segment ahead of the backward sweep,
@@ -2228,14 +2246,11 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
                     pa.tw = s.tw_x;
                     run_row(c, p.nx, ROW_ADJ, pa, nb, p.ny, st);
                     launch_sum_waves(gVw, nb, N, gV + (int64_t)i * N, st);
-                    pa.tw = s.tw_y;
                     if (i > 0) {
+                        pa.tw = s.tw_y;
                         pa.slice = i - 1;
                         pa.flags = PF_CONJ_PROP | PF_PROP_ALWAYS;
                         run_col(c, p.ny, COL_STEP, pa, nb, p.nx, st);
-                    } else {
-                        run_col(c, p.ny, COL_GRAD_PROBE, pa, nb, p.nx, st);
-                        launch_chi_finalize(chi_part, nb, tiles, chi_acc, st);
                     }
                 }
                 if (two && seg - 2 >= 0) {
@@ -2251,21 +2266,22 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
             // the side stream and the events exist before a capture uses them
             pot_stream(c);
             chunk_event(c, (size_t)(2 * nseg));
-            std::string key = graph_key_of(pa0, nb, S, nblk, ndet, partial, Iw, dtgt + (int64_t)start * ndet, dthr, -4);
-            const void* ptrs[] = {xseg, ckpt, gV, gVw, resid, sq + (int64_t)start * ndet, chi_part, chi_acc};
+            std::string key = graph_key_of(pa0, nb, S, nblk, ndet, partial, Iw, dtgt, dthr, -4);
+            const void* ptrs[] = {xseg, ckpt, gV, gVw, resid, sq};
             key.append((const char*)ptrs, sizeof(ptrs));
             key.append((const char*)&k, sizeof(k));
             run_graphed(c, key, body);
         } else {
             body();
         }
+        run_col(c, p.ny, COL_GRAD_PROBE, probe, nb, p.nx, st);
+        launch_chi_finalize(chi_part, nb, tiles, chi_acc, st);
+        CK(cudaMemcpyAsync(hsq.data() + (int64_t)start * ndet, sq, sizeof(double) * nb * ndet, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));  // the host wave table is refilled by the next batch
     }
     if (dV != gV)
         CK(cudaMemcpyAsync(dV, gV, sizeof(float) * slot, on_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
-    std::vector<double> hsq((size_t)np * ndet);
     double hchi[2];
-    CK(cudaMemcpyAsync(hsq.data(), sq, sizeof(double) * np * ndet, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(hchi, chi_acc, sizeof(double) * 2, cudaMemcpyDeviceToHost, st));
     tm.stop();
     double L = 0.0;

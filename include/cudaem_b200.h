@@ -204,6 +204,9 @@ int ms_last_probe_batch(const ms_ctx* ctx);
 /* Enables (1, the default) or disables (0) replaying each STEM probe batch from a captured
  * CUDA graph.  Disabled, every launch is issued directly; the results are identical. */
 ms_status ms_set_graphs(ms_ctx* ctx, int enable);
+/* Number of launch sequences the last call captured as graphs (those it replayed from earlier
+ * captures not counted).  The context keeps the eight used last. */
+int ms_last_graph_captures(const ms_ctx* ctx);
 /* Kernel form of the hot slice passes: 0 (default) the classic kernels, one block per tile
  * of rows or columns, launched slice by slice for CBED / TEM / STEM, while an uneven batch's grid
  * groups run in the persistent slice engine (form 2; groups of 2048 points slice by slice); 3 the
