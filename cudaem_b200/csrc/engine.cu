@@ -851,7 +851,7 @@ int choose_tile(ms_ctx* c, PassArgs pa, int nx, int ny, int nw, int nslices, cud
     if (c->tile_shape >= 0) return c->tile_shape;
     if ((!pa.tt && !pa.sV) || pa.variant == PASS_PIPELINED || nslices <= 0) return TILE_WIDE;
     char key[64];
-    // (2048-point steps on 32-thread teams, the gradient calls', are other kernels than the usual ones)
+    // (the adjoint's 2048-point steps, on 32-thread teams, are other kernels than the usual ones)
     std::snprintf(key, sizeof(key), "%d,%d,%d%s", nx, ny, nw, (nx == 2048 || ny == 2048) && !pa.tw64 ? ",32" : "");
     auto it = c->tile_choice.find(key);
     if (it != c->tile_choice.end()) return it->second;
@@ -2161,10 +2161,12 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
         upload(c, dtgt, target + (int64_t)start * ndet, sizeof(float) * nb * ndet, st);
         PassArgs pa = pass_args(s, adj, dwv, sV, slot, cond);
         pa.tt = sT;
-        // forward, recomputed and adjoint steps are those whose transforms the adjoint kernels share
-        pa.tw64 = nullptr;
         pa.l2_mode = l2_mode_for_waves(nb, N);
+        // The forward and recomputed steps are the forward call's, so that both compute the same
+        // intensities bit for bit; at 2048 points the adjoint steps alone run on the tiles, and choose them.
+        pa.tw64 = nullptr;
         pa.tile = choose_tile(c, pa, p.nx, p.ny, nb, S, st);
+        pa.tw64 = s.tw64;
         pa.det_thr = dthr;
         pa.ndet = ndet;
         pa.resid = resid;

@@ -90,7 +90,7 @@ struct PassArgs {
     const float4* short_x;    // twiddles of the short steps for rows and columns (fft.cuh), or null: not used
     const float4* short_y;
     const float2* tw64;       // those of 2048 points on teams of 64 threads, or null: the slice steps of
-                              // that length run on teams of 32 (gradient calls, whose bits stay)
+                              // that length run on teams of 32 (as the adjoint steps always do)
     const float2* prop_x;     // [nx] exp(i w (gx - g0x)^2)
     const float2* prop_y;     // [ny] exp(i w (gy - g0y)^2)
     const float2* prop;       // [kPropSets][ny][nx] full propagator P(k) including 1/N and the band limit (dithered)

@@ -1009,8 +1009,8 @@ static bool col_pipe(const PassArgs& a, int nwaves, int nx, cudaStream_t st)
 // The 2048-point slice steps (instantiated by the 2048-point unit only)
 //
 // Row step of 2048 points, one row per 64-thread block (team64_fft): k_row_tt's operations, on either
-// store (SV: a σV store)
-template <int MODE, bool SV>
+// store (SV: a σV store); KEEP_X: the transmitted wave also goes to PassArgs.xs (ROWF_KEEP_X)
+template <int MODE, bool SV, bool KEEP_X = false>
 __global__ void __launch_bounds__(64, 8) k_row_2048(PassArgs a)
 {
     constexpr int N = 2048;
@@ -1043,6 +1043,11 @@ __global__ void __launch_bounds__(64, 8) k_row_2048(PassArgs a)
             const uint64_t pol = l2_policy_trans(MODE);
 #pragma unroll
             for (int j = 0; j < 32; j++) v[j] = cmul(v[j], ld_nc_l2hint(tr + 64 * j, pol));
+        }
+        if constexpr (KEEP_X) {
+            float2* xr = opaque(a.xs) + ((size_t)b * ny + r) * N + t;
+#pragma unroll
+            for (int j = 0; j < 32; j++) xr[64 * j] = v[j];
         }
     }
     team64_fft<-1>(v, t, tw, scr, xch, sync);
@@ -1128,11 +1133,11 @@ __global__ void __launch_bounds__(64 * TC, 2) k_col_2048(PassArgs a, const __gri
     return true;
 }
 
-template <int MODE>
+template <int MODE, bool KEEP_X = false>
 static void row_2048(const PassArgs& a, int nwaves, int ny, cudaStream_t st)
 {
-    if (a.tt) launch_step(k_row_2048<MODE, false>, (unsigned)(nwaves * ny), 64, 0, st, a.chained != 0, a);
-    else launch_step(k_row_2048<MODE, true>, (unsigned)(nwaves * ny), 64, 0, st, a.chained != 0, a);
+    auto kern = a.tt ? k_row_2048<MODE, false, KEEP_X> : k_row_2048<MODE, true, KEEP_X>;
+    launch_step(kern, (unsigned)(nwaves * ny), 64, 0, st, a.chained != 0, a);
 }
 
 // The slice steps of small batches (short_fft), bound by latency: the slice's transmission and the
@@ -1283,6 +1288,8 @@ void row_dispatch(int op, const PassArgs& a, int nwaves, int ny, cudaStream_t st
         launch_step(kern, (unsigned)(nwaves * (ny / NL::ROWS)), NL::ROW_THREADS, nsm, st, a.chained != 0, a);
     };
     if (op == ROW_INV_T_FWD && (a.flags & PF_STORE_X)) {
+        if constexpr (N == 2048)
+            if (a.tw64) return row_2048<L2_DEFAULT, true>(a, nwaves, ny, st);
         if (narrow && a.tt) narrow_step(k_row_tt<N, L2_DEFAULT, NL, false, ROWF_KEEP_X>);
         else if (narrow) narrow_step(k_row_tt<N, L2_DEFAULT, NL, true, ROWF_KEEP_X>);
         else if (a.tt) wide_step(k_row_tt<N, L2_DEFAULT, L, false, ROWF_KEEP_X>);

@@ -39,3 +39,25 @@ def test_uneven_batch(ctx):
     outs, _ = cb.MulSimulator(ctx=ctx).executionMany(jobs)
     for (p, at), o in zip(jobs, outs):
         assert rel(o.image_intensity, orc.simulate_cbed(p, at)) < 1e-5
+
+
+@pytest.mark.parametrize("nx,ny,n_probe", [(2048, 128, 4), (128, 2048, 4), (2048, 2048, 1), (128, 128, 5)])
+def test_gradient_sees_the_forward_call_s_intensities(ctx, nx, ny, n_probe):
+    """At its own forward intensities the loss is what rounding the targets to float leaves, at every length
+    and on both slice stores (fewer than four probes read sigma V): at most half a unit in the last place
+    per intensity.  Gradients as far from the oracle's as at the other lengths (1e-4)."""
+    p, _ = wl.stem_sto(cells=(3, 3, 2), n=nx, nconf=1, scan=(1, 1), step=0.4, batch=0)
+    p.ny = ny
+    p.set_detectors([(0.0, 0.012), (0.025, 0.06)])
+    p.ckpt_interval = 2
+    rng = np.random.default_rng(nx + n_probe)
+    V = rng.uniform(0, 0.4, (5, ny, nx)).astype(np.float32)
+    xy = p.lx / 2 + rng.uniform(-1.0, 1.0, (n_probe, 2))
+    I = ctx.stem_forward_potential(p, V, 0.5, xy)
+    loss = ctx.stem_backward(p, V, 0.5, xy, I)[0]
+    assert loss <= np.sum((I.astype(float) * 2.0 ** -24) ** 2) * 1.0001
+    if nx * ny < 2048 * 2048:
+        T = (I * (1 + 0.05 * rng.standard_normal(I.shape))).astype(np.float32)
+        _, gV, g10, _ = ctx.stem_backward(p, V, 0.5, xy, T)
+        _, gVo, g10o, _ = orc.stem_backward(p, V, 0.5, xy, T)
+        assert rel(gV, gVo) < 1e-4 and abs(g10 - g10o) < 1e-4 * abs(g10o)
