@@ -827,6 +827,13 @@ int l2_mode_for_waves(int nwaves, int64_t N)
     return (double)nwaves * (double)N * sizeof(float2) <= 72.0 * 1024 * 1024 ? L2_WAVES_RESIDENT : L2_DEFAULT;
 }
 
+// A scan's batch shares one transmission slice: that stays in L2, or the waves do if they fit (64 probes of
+// 512 x 256, 20 slices: 6.70 -> 6.45 ms for 91 probes, 3 configurations).
+int l2_mode_for_scan(int nwaves, int64_t N)
+{
+    return l2_mode_for_waves(nwaves, N) == L2_WAVES_RESIDENT ? L2_WAVES_RESIDENT : L2_SHARED_T;
+}
+
 // Whether the slice steps of a batch are launched chained (launch_step): batches so small that the
 // launch latency between two steps shows, up to 2^19 wave pixels.  Per slice, plain and chained:
 // 1 x 256^2 6.74 and 5.84 us, 8 x 256^2 8.49 and 8.23, 1 x 512^2 11.56 and 10.54; but 1 x 1024^2
@@ -850,9 +857,13 @@ int choose_tile(ms_ctx* c, PassArgs pa, int nx, int ny, int nw, int nslices, cud
 {
     if (c->tile_shape >= 0) return c->tile_shape;
     if ((!pa.tt && !pa.sV) || pa.variant == PASS_PIPELINED || nslices <= 0) return TILE_WIDE;
+    if (nx == 2048 && ny == 2048 && pa.tw64) return TILE_WIDE;   // neither step has tiles to choose
     char key[64];
-    // (the adjoint's 2048-point steps, on 32-thread teams, are other kernels than the usual ones)
-    std::snprintf(key, sizeof(key), "%d,%d,%d%s", nx, ny, nw, (nx == 2048 || ny == 2048) && !pa.tw64 ? ",32" : "");
+    // Other kernels than the usual ones: the adjoint's 2048-point steps (32-thread teams), steps on a
+    // sigma V store, and scans whose transmission slice stays in L2.
+    std::snprintf(key, sizeof(key), "%d,%d,%d%s%s%s", nx, ny, nw,
+                  (nx == 2048 || ny == 2048) && !pa.tw64 ? ",32" : "", pa.tt ? "" : ",v",
+                  pa.l2_mode == L2_SHARED_T ? ",s" : "");
     auto it = c->tile_choice.find(key);
     if (it != c->tile_choice.end()) return it->second;
     if (c->profile) return TILE_WIDE;   // per-launch events would time the events
@@ -1448,7 +1459,7 @@ int batch_cap(ms_ctx* c, int64_t N)
 // Probe-batch autotuner: times one probe generation and two slice steps (row + column pass)
 // for each candidate batch size on the call's own grid and potentials, and keeps the size
 // with the highest probe*slice rate.  The choice is cached in the context per grid, slice
-// count and cap.  Candidates are powers of two from 32 to 256 within the memory cap.
+// count, cap and slice store.  Candidates are powers of two from 32 to 256 within the memory cap.
 int autotune_batch(ms_ctx* c, const ms_params& p, const Setup& s, const PassArgs& base, const WaveInfo& w0, int S,
                    int npos, int cap)
 {
@@ -1460,7 +1471,7 @@ int autotune_batch(ms_ctx* c, const ms_params& p, const Setup& s, const PassArgs
     // (the timed row steps read the slices: without a store there is nothing to time)
     if (cand.size() == 1 || c->profile || (!base.tt && !base.sV)) return cand.back();
     char key[96];
-    std::snprintf(key, sizeof(key), "%d,%d,%d,%d", p.nx, p.ny, std::min(S, 2), hi);
+    std::snprintf(key, sizeof(key), "%d,%d,%d,%d%s", p.nx, p.ny, std::min(S, 2), hi, base.tt ? "" : ",v");
     auto it = c->batch_choice.find(key);
     if (it != c->batch_choice.end()) return std::max(1, std::min(it->second, hi));
     cudaStream_t st = c->stream;
@@ -1479,6 +1490,7 @@ int autotune_batch(ms_ctx* c, const ms_params& p, const Setup& s, const PassArgs
     pa.waves = dwv;
     for (int rep = 0; rep < 2; rep++) {   // the first round warms up every candidate
         for (int b : cand) {
+            pa.l2_mode = l2_mode_for_scan(b, s.N);   // as the batch will run
             CK(cudaEventRecord(e0, st));
             pa.tw = s.tw_y;
             launch_col(p.ny, COL_PROBE_INV, pa, b, p.nx, st);
@@ -1728,11 +1740,7 @@ void sim_stem(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* out)
             const int nb = std::min(B, npos - start);
             CK(cudaMemcpyAsync(dwv, dwv_all + start, sizeof(WaveInfo) * nb, cudaMemcpyDeviceToDevice, st));
             PassArgs pa = pass_args(s, psi, dwv, sVs, plain ? 0 : slot, cond);
-            // one transmission slice serves the whole batch: it stays in L2, or the waves do if they fit
-            // (64 probes of 512 x 256, 20 slices: 6.70 -> 6.45 ms for 91 probes, 3 configurations)
-            pa.l2_mode = plain                                               ? L2_DEFAULT
-                         : l2_mode_for_waves(nb, N) == L2_WAVES_RESIDENT ? L2_WAVES_RESIDENT
-                                                                         : L2_SHARED_T;
+            pa.l2_mode = plain ? L2_DEFAULT : l2_mode_for_scan(nb, N);
             pa.tt = sT;
             if (!plain) {
                 pa.tile = choose_tile(c, pa, p.nx, p.ny, nb, S, st);

@@ -225,17 +225,20 @@ ms_status ms_set_pass_kernels(ms_ctx* ctx, int variant);   /* 0..3 */
  * bit 2 one warp per column (1024-point columns; swizzled tile and transposed propagator; takes
  * precedence over bit 1): 0 wide tiles (blocks of 8..16 rows or columns), 1 narrow rows, 2 narrow
  * columns, 3 both, 4 warp columns, 5 warp columns and narrow rows.  Narrow
- * tiles spread batches too small to fill the GPU over every SM.  The autotuner times the four
- * shapes on the call's own data the first time a grid and batch size are seen.  All shapes
- * compute the same operations bit for bit.  No reference counterpart (the reference's FFTs are
- * cuFFT plans). */
+ * tiles spread batches too small to fill the GPU over every SM.  The autotuner times the
+ * shapes on the call's own data the first time a grid, batch size and slice store are seen.  All shapes
+ * compute the same operations bit for bit.  Steps without tiles run as they are whatever the
+ * shape: those of 2048 points, except the gradient's adjoint steps, and, in HRTEM, ED and thickness
+ * calls, those of small batches (512 points: up to 2^19 wave pixels; 256 and 128: up to 2^18).  No
+ * reference counterpart (the reference's FFTs are cuFFT plans). */
 ms_status ms_set_tile_shape(ms_ctx* ctx, int shape);
 /* How CBED / TEM / STEM calls keep their slices between the potential kernel and the slice loop:
  * 1 (default) as the transmission function t = exp(iσV) (FP32 complex, formed once per pixel in
  * the potential kernel), 0 as σV (FP32, t formed in the row step from the same table).  Both give
  * the same values; the choice trades the store's size and traffic against row-step arithmetic. */
 ms_status ms_set_transmission_store(ms_ctx* ctx, int enable);
-/* Tile shape (the bit mask above) of the last CBED / TEM / STEM call's hot passes. */
+/* Tile shape (the bit mask above) chosen for the last CBED / TEM / STEM call; steps without tiles
+ * (above) do not use it. */
 int ms_last_tile_shape(const ms_ctx* ctx);
 /* JSON file that keeps the autotuner's choices (probe batch, tile shape) across contexts and
  * processes, keyed by device, grid and batch size; entries already in the file are loaded now.
@@ -257,7 +260,11 @@ ms_status ms_set_potential_overlap(ms_ctx* ctx, int enable);
  * the kernel records it and returns, and the call fails with MS_ERR_TIMEOUT; the context stays
  * usable.  MS_INJECT_ALLOC_FAIL makes every device allocation the context would make fail, as a
  * cudaMalloc that ran out of memory: the call fails with MS_ERR_OUT_OF_MEMORY and the context
- * stays usable.  MS_INJECT_NONE (0) switches injection off. */
+ * stays usable (unless the buffers it had yet to make are those a call can do without: the
+ * transmission store of ms_stem_forward_potential and ms_stem_backward, up to a quarter of the memory
+ * their other buffers leave, and the gradient's copy for V_on_device, up to a twentieth of the free
+ * memory.  The context keeps them, and frees them when another call needs the room).
+ * MS_INJECT_NONE (0) switches injection off. */
 enum { MS_INJECT_NONE = 0, MS_INJECT_WAIT_TIMEOUT = 1, MS_INJECT_ALLOC_FAIL = 2 };
 ms_status ms_set_fault_injection(ms_ctx* ctx, int what);
 
@@ -323,7 +330,9 @@ ms_status ms_projected_potential(ms_ctx* ctx, const ms_params* p, const ms_atoms
 /* Runs a convergent probe at each of `n_probe` positions (probe_xy = x0,y0,x1,y1,... in A)
  * through slices with the given phase arrays V[n_slices][ny][nx] (rad; t = exp(i V)), and
  * writes the annular-detector intensities I[n_probe][n_det].  z_init is the defocus shift
- * of the probe (slice_middle_z(0), wave_function.cuh:56). */
+ * of the probe (slice_middle_z(0), wave_function.cuh:56).  Device memory that a caller passes here or
+ * below is used on the context's stream, which does not wait for other streams: its contents must be
+ * complete before the call. */
 ms_status ms_stem_forward_potential(ms_ctx* ctx, const ms_params* p, const float* V, int n_slices,
                                     int V_on_device, double z_init, const double* probe_xy, int n_probe,
                                     float* I_out);
