@@ -23,7 +23,7 @@ CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CU_SOURCES = ["kernels.cu", "passes_128.cu", "passes_256.cu", "passes_512.cu", "passes_1024.cu", "passes_2048.cu",
-              "engine.cu", "noalloc.cu"]
+              "passes_2048_cols.cu", "engine.cu", "noalloc.cu"]
 CPP_SOURCES = ["host.cpp", "abi.cpp", "tune.cpp"]
 
 

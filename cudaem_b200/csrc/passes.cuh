@@ -8,7 +8,8 @@
 // (inverse cuFFT with the P load callback, propagation_function.cuh:41-48).
 // The probe is generated inside the first column pass and the CTF inside the
 // HRTEM column pass.  Every transform length is compiled in its own translation
-// unit (passes_<N>.cu), which instantiates row_dispatch<N> and col_dispatch<N>.
+// unit (passes_<N>.cu; 2048 points, the longest to compile, in two), which instantiates
+// row_dispatch<N> and col_dispatch<N>.
 #pragma once
 #include <cuda.h>
 
@@ -1121,9 +1122,9 @@ __global__ void __launch_bounds__(64 * TC, 2) k_col_2048(PassArgs a, const __gri
 #pragma unroll
     for (int j = 0; j < 32; j++) st_l2hint(cp + j * cs, v[j], pol);
 }
-[[maybe_unused]] static bool col_2048(const PassArgs& a, int nwaves, int nx, cudaStream_t st)
+template <int TC>
+static bool col_2048(const PassArgs& a, int nwaves, int nx, cudaStream_t st)
 {
-    constexpr int TC = kCol2048;
     if (((uintptr_t)a.psi & 15) != 0) return false;
     CUtensorMap map;
     if (!encode_wave_tile_map(&map, a.psi, nx, (int64_t)nwaves * 2048, 2 * TC, 256)) return false;
@@ -1262,6 +1263,18 @@ static bool col_short(const PassArgs& a, int nwaves, int nx, cudaStream_t st)
     }
 }
 
+// The row step for an L2 mode.  (At 2048 points the 64-thread teams carry the modes; this form serves the
+// calls without their tables, on the default one.)
+template <int N, class L, bool SV>
+static void (*row_step_kernel(int l2_mode))(PassArgs)
+{
+    if constexpr (N != 2048) {
+        if (l2_mode == L2_WAVES_RESIDENT) return k_row_tt<N, L2_WAVES_RESIDENT, L, SV>;
+        if (l2_mode == L2_SHARED_T) return k_row_tt<N, L2_SHARED_T, L, SV>;
+    }
+    return k_row_tt<N, L2_DEFAULT, L, SV>;
+}
+
 template <int N>
 void row_dispatch(int op, const PassArgs& a, int nwaves, int ny, cudaStream_t st)
 {
@@ -1288,12 +1301,15 @@ void row_dispatch(int op, const PassArgs& a, int nwaves, int ny, cudaStream_t st
         launch_step(kern, (unsigned)(nwaves * (ny / NL::ROWS)), NL::ROW_THREADS, nsm, st, a.chained != 0, a);
     };
     if (op == ROW_INV_T_FWD && (a.flags & PF_STORE_X)) {
-        if constexpr (N == 2048)
-            if (a.tw64) return row_2048<L2_DEFAULT, true>(a, nwaves, ny, st);
-        if (narrow && a.tt) narrow_step(k_row_tt<N, L2_DEFAULT, NL, false, ROWF_KEEP_X>);
-        else if (narrow) narrow_step(k_row_tt<N, L2_DEFAULT, NL, true, ROWF_KEEP_X>);
-        else if (a.tt) wide_step(k_row_tt<N, L2_DEFAULT, L, false, ROWF_KEEP_X>);
-        else wide_step(k_row_tt<N, L2_DEFAULT, L, true, ROWF_KEEP_X>);
+        if constexpr (N == 2048) {
+            if (!a.tw64) throw MsError(MS_ERR_INTERNAL, "the 2048-point step that keeps its wave needs the 64-thread tables");
+            row_2048<L2_DEFAULT, true>(a, nwaves, ny, st);
+        } else {
+            if (narrow && a.tt) narrow_step(k_row_tt<N, L2_DEFAULT, NL, false, ROWF_KEEP_X>);
+            else if (narrow) narrow_step(k_row_tt<N, L2_DEFAULT, NL, true, ROWF_KEEP_X>);
+            else if (a.tt) wide_step(k_row_tt<N, L2_DEFAULT, L, false, ROWF_KEEP_X>);
+            else wide_step(k_row_tt<N, L2_DEFAULT, L, true, ROWF_KEEP_X>);
+        }
         return;
     }
     if (op == ROW_ADJ) {
@@ -1314,27 +1330,11 @@ void row_dispatch(int op, const PassArgs& a, int nwaves, int ny, cudaStream_t st
             return;
         }
     }
-    if (op == ROW_INV_T_FWD && a.tt) {
-        if (narrow)
-            narrow_step(a.l2_mode == L2_WAVES_RESIDENT ? k_row_tt<N, L2_WAVES_RESIDENT, NL>
-                        : a.l2_mode == L2_SHARED_T     ? k_row_tt<N, L2_SHARED_T, NL>
-                                                       : k_row_tt<N, L2_DEFAULT, NL>);
-        else
-            wide_step(a.l2_mode == L2_WAVES_RESIDENT ? k_row_tt<N, L2_WAVES_RESIDENT>
-                      : a.l2_mode == L2_SHARED_T     ? k_row_tt<N, L2_SHARED_T>
-                                                     : k_row_tt<N, L2_DEFAULT>);
-        return;
-    }
     if (op == ROW_INV_T_FWD) {
-        // the row step on a σV store
-        if (narrow)
-            narrow_step(a.l2_mode == L2_WAVES_RESIDENT ? k_row_tt<N, L2_WAVES_RESIDENT, NL, true>
-                        : a.l2_mode == L2_SHARED_T     ? k_row_tt<N, L2_SHARED_T, NL, true>
-                                                       : k_row_tt<N, L2_DEFAULT, NL, true>);
-        else
-            wide_step(a.l2_mode == L2_WAVES_RESIDENT ? k_row_tt<N, L2_WAVES_RESIDENT, L, true>
-                      : a.l2_mode == L2_SHARED_T     ? k_row_tt<N, L2_SHARED_T, L, true>
-                                                     : k_row_tt<N, L2_DEFAULT, L, true>);
+        if (narrow && a.tt) narrow_step(row_step_kernel<N, NL, false>(a.l2_mode));
+        else if (narrow) narrow_step(row_step_kernel<N, NL, true>(a.l2_mode));
+        else if (a.tt) wide_step(row_step_kernel<N, L, false>(a.l2_mode));
+        else wide_step(row_step_kernel<N, L, true>(a.l2_mode));
         return;
     }
     const dim3 grid((unsigned)(nwaves * (ny / L::ROWS))), block(L::ROW_THREADS);
@@ -1364,7 +1364,7 @@ void col_dispatch(int op, const PassArgs& a, int nwaves, int nx, cudaStream_t st
     // the hot column step reads its tile through the tensor memory accelerator
     if (op == COL_STEP && a.variant != PASS_PIPELINED && !(a.flags & PF_FILTER_AUX)) {
         if constexpr (N == 2048)
-            if (a.tw64 && !(a.flags & PF_CONJ_PROP) && col_2048(a, nwaves, nx, st)) return;
+            if (a.tw64 && !(a.flags & PF_CONJ_PROP) && col_2048<kCol2048>(a, nwaves, nx, st)) return;
         if ((a.tile & TILE_WARP_COLS) && col_step_warp<N>(a, nwaves, nx, st)) return;
         if ((a.tile & TILE_NARROW_COLS) && col_step_tma<N, NarrowLayout<N>>(a, nwaves, nx, st)) return;
         if (col_step_tma<N>(a, nwaves, nx, st)) return;
