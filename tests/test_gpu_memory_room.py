@@ -16,6 +16,7 @@ sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
 
 import cases  # noqa: E402
 import cudaem_b200 as cb  # noqa: E402
+from cudaem_b200 import _abi as abi  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 MB = 1 << 20
@@ -82,6 +83,27 @@ def test_forward_keeps_its_route_and_yields_its_store(fixed):
         # one probe on host slices that need nearly all of the memory: the store gives way
         vacuum = fixed.stem_forward_potential(p2, big, 0.5, xy[:1])
     assert np.allclose(vacuum, few, rtol=1e-3)   # empty slices keep the band-limited probe
+
+
+def test_forward_without_room_for_its_store(fixed):
+    """Above a quarter of the free memory, or when the allocation fails, t is formed probe by probe: the same
+    values."""
+    p, _ = cases.stem_small(n=128)
+    p.probe_batch = 2
+    free = 300 * MB
+    V = phases(p, int(0.4 * free) // (8 * 128 * 128))
+    xy = probes(p, 4)
+    forward(fixed, p, V[:2], xy[:3])
+    with only_free(free):
+        tight, n_tight = forward(fixed, p, V, xy)
+    few = V[:40]
+    fixed.set_fault_injection(abi.MS_INJECT_ALLOC_FAIL)
+    failed, n_failed = forward(fixed, p, few, xy)
+    fixed.set_fault_injection(abi.MS_INJECT_NONE)
+    with_store, n_store = forward(fixed, p, few, xy)
+    assert np.array_equal(failed, with_store) and n_failed == n_store - 1
+    roomy, n_roomy = forward(fixed, p, V, xy)
+    assert np.array_equal(tight, roomy) and n_tight == n_roomy - 1
 
 
 def test_backward_keeps_its_batch(fixed):
