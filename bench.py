@@ -336,8 +336,9 @@ def extras(ctx, pass_kernels: int = 0):
 
     out["uneven_batch"] = dict(workload="64 CBED instances drawn from seed 42: grids 256^2..2048^2, 10-200 slices "
                                         "of SrTiO3 or Si, 80-300 kV, 10-30 mrad, one phonon configuration each; "
-                                        "every grid group in one persistent slice-engine launch (the default); "
-                                        "latency = the device clock at which an instance's last wave was done",
+                                        "the default: grid groups up to 1024^2 in one persistent slice-engine launch "
+                                        "each, latency = the device clock at which an instance's last wave was "
+                                        "done; 2048^2 slice by slice, latency = its completion event",
                                **uneven(0))
     out["uneven_batch"]["per_slice_launches"] = uneven(3)
     out["uneven_batch"]["per_slice_launches"]["note"] = ("one row and one column launch per slice and grid group, "

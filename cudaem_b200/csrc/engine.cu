@@ -846,12 +846,12 @@ bool chain_steps(const ms_ctx* c, int nwaves, int64_t N)
 
 // Tile shape of the hot passes (row step on the transmission store, column step) for a batch of
 // nw waves on an nx x ny grid: forced by ms_set_tile_shape, else the fastest of the four
-// combinations of wide and narrow row and column tiles, timed on the call's own transmission store
+// combinations of wide and narrow row and column tiles, timed on the call's own slice store
 // (slices 0..nslices-1), wave descriptors and wave buffer, before the wave is set up.  Each timing covers enough slice
 // steps for about 2 ms of work (at least two), so that a single small wave is timed above the
 // event resolution; a shape's time is the best of two timed rounds after one untimed round.  The
-// choice is kept per device, grid and batch size in the context and in the JSON cache file when
-// one is set.  Under a profiler the timings are distorted: a cache file written by a plain run
+// choice is kept per device, grid, batch size and slice store in the context and in the JSON cache file
+// when one is set.  (It also stands for batches of that size whose steps have no tiles.)  Under a profiler the timings are distorted: a cache file written by a plain run
 // keeps the choice of a profiled run the same.
 int choose_tile(ms_ctx* c, PassArgs pa, int nx, int ny, int nw, int nslices, cudaStream_t st)
 {
@@ -1013,7 +1013,8 @@ EngineArgs engine_plan(ms_ctx* c, const std::vector<int>& ns, int slice0, int N,
 // otherwise the batch runs slice by slice.
 bool engine_fits(const ms_ctx* c, int nx, int ny, int flags, bool uneven = false)
 {
-    // (2048-point groups of an uneven batch: the per-slice steps on 64-thread teams are faster)
+    // (2048-point groups of an uneven batch take the steps on 64-thread teams, as a CBED call alone does, so
+    // that both give the same values; two instances of 2048^2: 15.8 ms slice by slice, 20.4 in the engine)
     const bool wanted = c->pass_variant == PASS_ENGINE || (uneven && c->pass_variant == PASS_CLASSIC && nx < 2048);
     return wanted && nx == ny && tensor_maps_available() &&
            !(flags & (PF_STORE_X | PF_FILTER_AUX | PF_VACUUM_BEYOND | PF_PROP_ALWAYS | PF_TILT_INCIDENT));
@@ -2568,7 +2569,10 @@ void sim_many(ms_ctx* c, int n, const ms_params* ps, const ms_atoms* as, ms_outp
                 pa.exptab = ex;
                 pa.grid = in[G.inst.front()].gd;
                 pa.err = c->d_err;
-                pa.tile = TILE_NARROW_ROWS;   // the faster row step at every length on batches
+                // narrow rows: the fastest shape at 256 and 1024 points, rectangles among them, or within
+                // 1 % of it (ten instances of 1024^2: 22.9 ms, wide 23.4, narrow columns 24.3, both 23.8; two
+                // of 512^2: 2.23, wide 2.59, both 2.11)
+                pa.tile = TILE_NARROW_ROWS;
                 pa.tw64 = twiddles64(c, G.nx, G.ny);
                 pa.tw = twiddles(c, G.nx);
                 launch_row(G.nx, ROW_INV_T_FWD, pa, nact, G.ny, G.s);
