@@ -2,7 +2,6 @@
 #pragma once
 #include <cuda_runtime.h>
 
-#include <initializer_list>
 #include <map>
 #include <string>
 #include <vector>
@@ -87,9 +86,8 @@ struct ms_ctx {
     bool has(const std::string& name, size_t bytes) const;   // held already, at this size or larger
     void return_spares();   // a call begins: none is in use
     bool drop_spares();     // frees those not in use; false: there were none
-    // Bytes that free_mem() does not count, held under these names by earlier calls: a size chosen by
-    // free_mem() + held() is the same on every call.
-    size_t held(std::initializer_list<const char*> names) const;
+    // Bytes that free_mem() does not count, held under these names by earlier calls.
+    size_t held(const std::vector<const char*>& names) const;
     void release_all();
 
     // Free device memory as cudaMemGetInfo reports it, and the spare buffers that are not in use.  The

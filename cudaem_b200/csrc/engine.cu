@@ -118,7 +118,7 @@ bool ms_ctx::drop_spares()
     return freed;
 }
 
-size_t ms_ctx::held(std::initializer_list<const char*> names) const
+size_t ms_ctx::held(const std::vector<const char*>& names) const
 {
     size_t sum = 0;
     for (const char* n : names) {
@@ -1070,6 +1070,36 @@ size_t free_budget(ms_ctx* c)
     return (size_t)(c->free_mem() * 0.6);
 }
 
+// How many waves or configurations, at most `cap`, run at once when each takes `bytes` of the named
+// buffers: 60 % of the free memory's worth.  What the buffers hold already counts as free for them, so a
+// repeated call is split as the first one was; what they have to grow by fits 60 % of what is free.
+struct PerUnit {
+    std::vector<const char*> names;
+    size_t bytes;
+};
+int units_that_fit(ms_ctx* c, const std::vector<PerUnit>& bufs, int cap)
+{
+    const double free = (double)c->free_mem();
+    double total = free;
+    std::vector<double> held;
+    for (const PerUnit& b : bufs) {
+        held.push_back((double)c->held(b.names));
+        total += held.back();
+    }
+    auto fits = [&](int n) {
+        double need = 0.0, growth = 0.0;
+        for (size_t i = 0; i < bufs.size(); i++) {
+            const double bytes = (double)bufs[i].bytes * n;
+            need += bytes;
+            growth += std::max(0.0, bytes - held[i]);
+        }
+        return need <= 0.6 * total && growth <= 0.6 * free;
+    };
+    int n = cap;
+    while (n > 1 && !fits(n)) n--;
+    return n;
+}
+
 void copy_out(ms_ctx* c, float* dst, const float* src, int64_t n, int on_dev)
 {
     CK(cudaMemcpyAsync(dst, src, sizeof(float) * n, on_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
@@ -1842,10 +1872,13 @@ void sim_thickness(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* 
     // `chunk` stored slices at once.  So the slice loop's chain of dependent launches is two per
     // slice instead of four for every configuration, and the image transforms run as full batches
     // (256^2, 24 slices, 2 configurations: 1697 us per call before, 875 us so, 746 us with short chained steps).
-    const size_t per_conf = (size_t)estimate_slices(p, a) * N * 8 + (size_t)N * 8 * 2 + (size_t)a.n * 40 +
-                            fine_bytes_per_conf(p, a);
-    const size_t budget = (size_t)(0.6 * (double)(c->free_mem() + c->held({"sT", "psi", "thick_aux"})));
-    const int gsize = (int)std::max<size_t>(1, std::min<size_t>(cs.confs.size(), budget / per_conf));
+    const std::vector<PerUnit> per_conf = {
+        {{"sT"}, (size_t)estimate_slices(p, a) * N * 8},
+        {{"psi"}, (size_t)N * 8},
+        {{"thick_aux"}, (size_t)N * 8},
+        {{"sp_xd", "sp_yd", "sp_zd", "sp_keys", "sp_keys2", "sp_vals", "sp_vals2", "sp_ax", "sp_ay", "sp_aw", "sp_ae",
+          "sp_az", "sp_fine_tab"}, (size_t)a.n * 40 + fine_bytes_per_conf(p, a)}};
+    const int gsize = units_that_fit(c, per_conf, (int)cs.confs.size());
     for (size_t g0 = 0; g0 < cs.confs.size(); g0 += gsize) {
         const std::vector<int> confs(cs.confs.begin() + g0, cs.confs.begin() + std::min(cs.confs.size(), g0 + gsize));
         SpecGroup g = build_specimen(c, p, A, confs, s.ph);
@@ -1853,9 +1886,10 @@ void sim_thickness(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* 
         const int64_t slot = (int64_t)g.S_cap * N;
         float2* sT = (float2*)c->buf("sT", sizeof(float2) * slot * nw);
         run_potential(c, with_transmission(pot_args(p, s, A, g, nullptr, slot, 0, g.S_cap, 0), sT, s), nw, st);
+        float2* psi = (float2*)c->buf("psi", sizeof(float2) * N * nw);
         // filtered spectra of a chunk of slices, at most 256 MB (they are read back from L2 when they
         // fit) and a sixteenth of the free memory, or one slice
-        const int64_t room = std::min<int64_t>(256ll << 20, (int64_t)((c->free_mem() + c->held({"psi", "thick_aux"})) / 16));
+        const int64_t room = std::min<int64_t>(256ll << 20, (int64_t)((c->free_mem() + c->held({"thick_aux"})) / 16));
         const int chunk = (int)std::max<int64_t>(1, std::min<int64_t>(nf, room / (8 * N * nw)));
         // the waves' descriptors, then one per stored slice (only their weight is read)
         std::vector<WaveInfo> wv((size_t)nw + chunk);
@@ -1869,7 +1903,6 @@ void sim_thickness(ms_ctx* c, const ms_params& p, const ms_atoms& a, ms_output* 
         }
         WaveInfo* dwv = (WaveInfo*)c->buf("waves", sizeof(WaveInfo) * wv.size());
         upload(c, dwv, wv.data(), sizeof(WaveInfo) * wv.size(), st);
-        float2* psi = (float2*)c->buf("psi", sizeof(float2) * N * nw);
         float2* aux = (float2*)c->buf("thick_aux", sizeof(float2) * N * nw * chunk);
         PassArgs pa = pass_args(s, psi, dwv, nullptr, slot, cond);
         pa.l2_mode = l2_mode_for_waves(nw, N);
@@ -2117,13 +2150,15 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
     upload(c, dthr, thr.data(), sizeof(float) * 2 * ndet, st);
     const int k = p.ckpt_interval;
     const int nseg = (S + k - 1) / k;
-    // probes per batch: adjoint wave, forward wave, one segment of transmitted waves and the
-    // checkpoints must fit the memory budget
-    const size_t per_wave = (size_t)N * 8 * (2 + 2 * (size_t)k + (size_t)(nseg - 1)) + (size_t)N * 4;
-    int B = p.probe_batch > 0 ? p.probe_batch : 256;
-    const size_t room = c->free_mem() + c->held({"adj_psi", "adj_xseg", "adj_ckpt", "adj_dVw", "adj_dV"});
-    B = (int)std::max<size_t>(1, std::min<size_t>((size_t)B, (size_t)(0.6 * (double)room) / per_wave));
-    B = std::min(B, np);
+    float* gV = !on_dev ? (float*)c->buf("adj_dV", sizeof(float) * slot) : nullptr;
+    // probes per batch: adjoint wave, forward wave, two segments of transmitted waves, the
+    // checkpoints and the gradient's planes must fit the memory budget
+    const int B = units_that_fit(c,
+                                 {{{"adj_psi"}, (size_t)N * 16},
+                                  {{"adj_xseg"}, (size_t)N * 16 * k},
+                                  {{"adj_ckpt"}, (size_t)N * 8 * (nseg - 1)},
+                                  {{"adj_dVw"}, (size_t)N * 4}},
+                                 std::min(np, p.probe_batch > 0 ? p.probe_batch : 256));
     const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>(64, N / 4096));
     const int tiles = col_tiles(p.ny, p.nx);
     float2* adj = (float2*)c->buf("adj_psi", sizeof(float2) * N * B);
@@ -2139,7 +2174,6 @@ void sim_stem_backward(ms_ctx* c, const ms_params& p, const float* V, int S, int
     double* chi_part = (double*)c->buf("adj_chi_part", sizeof(double) * B * tiles * 2);
     double* chi_acc = (double*)c->buf("adj_chi", sizeof(double) * 2);
     WaveInfo* dwv = (WaveInfo*)c->buf("waves", sizeof(WaveInfo) * B);
-    float* gV = !on_dev ? (float*)c->buf("adj_dV", sizeof(float) * slot) : nullptr;
     float2* sT = caller_transmission(c, s, sV, slot, np);
     // The batch's launches replay from a graph when they hold none of the caller's pointers: on the
     // transmission store, with the gradient summed in the context's memory and copied out at the end

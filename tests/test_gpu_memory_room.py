@@ -106,21 +106,40 @@ def test_forward_without_room_for_its_store(fixed):
     assert np.array_equal(tight, roomy) and n_tight == n_roomy - 1
 
 
+def gradient(ctx, p, V, xy, n):
+    target = np.zeros((len(xy), p.n_det), np.float32)
+    gV = torch.empty_like(V)
+    loss, g10, g30 = C.c_double(), C.c_double(), C.c_double()
+    cp = p.c()
+    ctx.check(cb.lib().ms_stem_backward(
+        ctx.handle, C.byref(cp), fptr(V), n, 1, 0.5, xy.ctypes.data_as(C.POINTER(C.c_double)), len(xy),
+        target.ctypes.data_as(C.POINTER(C.c_float)), C.byref(loss), fptr(gV), C.byref(g10), C.byref(g30)))
+    return loss.value, gV[:n].cpu().numpy(), ctx.last_launch_count
+
+
+def test_gradient_after_one_of_another_checkpoint_interval(fixed):
+    """Checkpoints of every slice leave one buffer large that another interval hardly uses: what it holds is
+    not room for the other buffers."""
+    p, _ = cases.stem_small(n=256)
+    p.set_detectors([(0.0, 0.012)])
+    V, xy = phases(p, 64), probes(p, 24)
+    gradient(fixed, p, V, xy, 9)
+    out = []
+    with only_free(600 * MB):
+        for k in (1, 32, 1, 8):
+            p.ckpt_interval = k
+            out.append(gradient(fixed, p, V, xy, 64))
+    assert all(abs(o[0] - out[0][0]) <= 1e-12 * out[0][0] and np.array_equal(o[1], out[0][1]) for o in out)
+
+
 def test_backward_keeps_its_batch(fixed):
     p, _ = cases.stem_small(n=256)
     p.set_detectors([(0.0, 0.012)])
     p.ckpt_interval = 8
     V, xy = phases(p, 64), probes(p, 24)
-    target = np.zeros((24, 1), np.float32)
-    gV = torch.empty_like(V)
 
     def call(n):
-        loss, g10, g30 = C.c_double(), C.c_double(), C.c_double()
-        cp = p.c()
-        fixed.check(cb.lib().ms_stem_backward(
-            fixed.handle, C.byref(cp), fptr(V), n, 1, 0.5, xy.ctypes.data_as(C.POINTER(C.c_double)), len(xy),
-            target.ctypes.data_as(C.POINTER(C.c_float)), C.byref(loss), fptr(gV), C.byref(g10), C.byref(g30)))
-        return loss.value, gV.cpu().numpy(), fixed.last_launch_count
+        return gradient(fixed, p, V, xy, n)
 
     call(9)
     with only_free(400 * MB):   # room for about 18 of the 24 probes
